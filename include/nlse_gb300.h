@@ -185,7 +185,9 @@ int nlse_solver_query(nlse_solver *s, int *idle);
 int nlse_solver_stream(nlse_solver *s, void **stream);
 /* Steps per captured CUDA graph (default 8; 0 disables graphs). */
 int nlse_solver_set_graph_steps(nlse_solver *s, int steps);
-/* Number of kernel launches one RK4 step enqueues. */
+/* Number of kernel launches one RK4 step takes stage by stage.  1D solves
+ * run several whole steps per launch where that is faster (knob "seg1d") and
+ * then enqueue fewer. */
 int nlse_solver_launches_per_step(const nlse_solver *s);
 /* Bytes of device memory held by the solver. */
 long long nlse_solver_device_bytes(const nlse_solver *s);
@@ -285,10 +287,10 @@ int nlse_take_steps_noalloc(const nlse_problem *p, const double *dUr, const doub
  *                  faces' own lo, K and V in face-indexed arrays that the
  *                  face kernel reads instead of the strided x faces; 0: the
  *                  full arrays.  Same bits.
- *   "small1d.max_points"  FP32 and mixed 1D solves of at most this many
- *                  points (default 2048, 0 = never, at most 65536) run each
- *                  chunk in single-block launches instead of a launch per
- *                  pass.  Same bits.
+ *   "small1d.max_points"  with "seg1d" 0, FP32 and mixed 1D solves of at
+ *                  most this many points (default 2048, 0 = never, at most
+ *                  65536) run each chunk in single-block launches instead of
+ *                  a launch per pass.  Same bits.
  *   "wide.z2"      1 (default): the mixed-precision 3D interior kernel (TMA
  *                  staging, both methods) advances two z planes per
  *                  iteration (one barrier and plane wait per two points);
@@ -314,12 +316,11 @@ int nlse_take_steps_noalloc(const nlse_problem *p, const double *dUr, const doub
  *                  layout-conversion kernels of nlse_solver_upload /
  *                  _download and the one-shot calls; 0: always staged
  *                  through device copies.  Same bits.
- *   "seg1d"        1 (default): 1D grids (BC 1-3) above
- *                  "small1d.max_points" take the staged-segment stage
- *                  kernels (one launch per stage, 2SHOC's D in shared
- *                  memory): 2SHOC in FP32 and mixed at every size, FP64
- *                  and CD below 2^22 points; 0: the gather kernels.  Same
- *                  bits.
+ *   "seg1d"        1 (default): 1D grids run several whole RK4 steps per
+ *                  launch, the points in registers (FP64 up to 2^16 points;
+ *                  above, BC 1-3 below 2^22 points take one staged-segment
+ *                  launch per stage); 0: the gather kernels.  Same bits
+ *                  (NLSE_FLAG_FMA: to rounding).
  * ---------------------------------------------------------------------- */
 int nlse_tune_set(const char *key, long long value);
 int nlse_tune_get(const char *key, long long *value);

@@ -28,11 +28,11 @@ cudaError_t launch_one(const Geom& g, const Consts<R>& c, const ExactStageArgs<R
   if (kernel_kind == KERNEL_TILED && tiled_supported(g, DIM)) {
     return tiled::launch_exact<R, DIM, METHOD, BC, VAR>(g, c, a, stage, st);
   }
-  // 1D grids: staged segments, one launch per stage.  FP32 2SHOC at every
-  // size (1.4-1.75x the D-scratch form), the rest below 2^22 points (FP64,
-  // bound by FP64 issue, and CD gain nothing on larger grids)
-  if constexpr (DIM == 1 && BC != 4) {
-    if (seg1d_exact_path(g, METHOD, BC, kernel_kind, sizeof(R) == 4))
+  // FP64 1D grids above the step kernel's limit (kern_step1d.cuh): staged
+  // segments, one launch per stage, below 2^22 points (bound by FP64 issue,
+  // larger grids gain nothing)
+  if constexpr (DIM == 1 && BC != 4 && sizeof(R) == 8) {
+    if (seg1d_exact_path(g, METHOD, BC, kernel_kind, false))
       return seg1d::launch_exact<R, METHOD, BC, VAR>(g, c, a, stage, st, wide::g_pdl != 0);
   }
   // FP32 on 2D grids: the single-pass tile kernel (2SHOC 1.4-1.5x the

@@ -2,7 +2,6 @@
 #include "kern_gather.cuh"
 #include "kern_tiled.cuh"
 #include "kern_wide.cuh"
-#include "kern_seg1d.cuh"
 #include "kern_wide2d.cuh"
 #include "nlse_launch.h"
 
@@ -25,8 +24,9 @@ int g_z2 = 1;
 int g_wide_ty = 8;
 // 2D grids (BC 1-3): one single-pass stage kernel per stage (kern_wide2d.cuh)
 int g_wide2d = 1;
-// 1D grids (BC 1-3) above the single-block size: one staged-segment launch
-// per stage (kern_seg1d.cuh), same bits as the gather kernels
+// 1D grids: whole steps in registers (kern_step1d.cuh; FP64 above its limit:
+// one staged-segment launch per stage, kern_seg1d.cuh), same bits as the
+// gather kernels
 int g_seg1d = 1;
 }
 namespace wide2d {
@@ -38,12 +38,6 @@ static cudaError_t launch_one(const Geom& g, const Consts<float>& c, const Mixed
                               int stage, cudaStream_t st, int kernel_kind) {
   if (DIM == 2 && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_wide2d)
     return wide2d::launch<METHOD, BC == 4 ? 1 : BC>(g, a, c, stage, st, wide::g_pdl != 0);
-  // 1D: 2SHOC always (one launch instead of D then F: 1.2-1.7x); CD, one
-  // gather launch already, below 2^22 points (1.1x at 2^20 points, 0.8x at
-  // 2^24 where the gather kernel keeps more loads in flight)
-  if (DIM == 1 && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_seg1d &&
-      (METHOD == 2 || g.n < (1LL << 22)))
-    return seg1d::launch<METHOD, BC == 4 ? 1 : BC>(g, a, c, stage, st, wide::g_pdl != 0);
   if (kernel_kind == KERNEL_TILED && tiled_supported(g, DIM) && DIM == 3 && BC != 4) {
     tiled::MixedPol::Args A{a, c, stage, tiled::error_word()};
     return wide::launch<METHOD, BC == 4 ? 1 : BC>(g, A, st);

@@ -198,25 +198,10 @@ __device__ __forceinline__ void segment_exact(const Geom& g, const Consts<R>& c,
   }
 }
 
-// Single-solve stage kernels: one CTA per segment of 256 points (one point
-// per thread), launched with PDL like the other stage kernels.
+// Single-solve stage kernel (FP64 grids above the step kernel's limit,
+// kern_step1d.cuh): one CTA per segment of 256 points (one point per thread),
+// launched with PDL like the other stage kernels.
 constexpr int SOLO_SEG = 256;
-
-template <int METHOD, int BC>
-__global__ void __launch_bounds__(NT) stage1d(Geom g, Consts<float> c, IO io, int stage) {
-  __shared__ Smem<SOLO_SEG> sm;
-  pdl_trigger();  // the next kernel may launch; it waits for this one
-  pdl_wait();     // the previous kernel's output
-  segment<METHOD, BC, SOLO_SEG>(g, c, io, stage, blockIdx.x, sm);
-}
-
-template <int METHOD, int BC>
-cudaError_t launch(const Geom& g, const MixedStageArgs& a, const Consts<float>& c, int stage,
-                   cudaStream_t st, bool pdl) {
-  const IO io{a.hi_in, a.lo_in, a.e_in, a.V, a.K, a.e_out, a.hi_out, a.lo_out};
-  return launch_k(stage1d<METHOD, BC>, dim3((unsigned)segments<SOLO_SEG>(g.n)), dim3(NT), 0, st,
-                  pdl, g, c, io, stage);
-}
 
 template <typename R, int METHOD, int BC, int VAR = 0>  // VAR: as exact::gather_stage
 __global__ void __launch_bounds__(NT)

@@ -73,10 +73,11 @@ static int g_default_graph_steps = 8;
 // the layout-conversion kernels in place, over the host link, instead of
 // being copied into a device staging buffer first.
 static int g_zero_copy = 1;
-// FP32 and mixed 1D solves of at most this many points run each chunk in
-// single-block launches (0: never).  At the 1024-point configuration this
-// runs 2.0-2.6x faster than a launch per pass; FP64 does not gain (one SM's
-// FP64 rate is the limit there) and keeps the stage launches.
+// With the step kernel off ("seg1d" 0), FP32 and mixed 1D solves of at most
+// this many points run each chunk in single-block launches (0: never).  At
+// the 1024-point configuration this runs 2.0-2.6x faster than a launch per
+// pass; FP64 does not gain (one SM's FP64 rate is the limit there) and keeps
+// the stage launches.
 static long long g_small1d_max = 2048;
 
 extern "C" int nlse_tune_set(const char* key, long long value) {
@@ -361,6 +362,7 @@ struct nlse_solver {
   // exact precisions
   void *psi, *K, *ya, *yb, *V;
   void* dsc;  // 2SHOC on the gather path: D scratch (C2<R> or float2 per point)
+  int flip;   // psi and ya are swapped (step launches write the state to the other buffer)
   // mixed precision
   float2 *hi[2], *lo[2], *mK, *da, *db, *dc, *fq;
   float4* gh;
@@ -761,10 +763,47 @@ static int run_small1d(nlse_solver* s, long long nsteps) {
   return NLSE_OK;
 }
 
+// 1D solves: several RK4 steps per launch, in registers (kern_step1d.cuh).
+static int run_step1d(nlse_solver* s, const Step1dShape& sh, long long nsteps) {
+  const nlse_problem& p = s->prob;
+  while (nsteps > 0) {
+    const int m = nsteps < sh.steps ? (int)nsteps : sh.steps;
+    cudaError_t e;
+    if (p.precision == NLSE_PREC_MIXED) {
+      const int c = s->cur;
+      e = launch_step1d_mixed(s->g, p.method, p.bc, s->cf, s->hi[c], s->lo[c], s->Vf,
+                              s->hi[1 - c], s->lo[1 - c], sh, m, s->stream);
+      s->cur = 1 - c;
+    } else {
+      if (p.precision == NLSE_PREC_SINGLE)
+        e = launch_step1d_exact<float>(s->g, p.method, p.bc, s->cf, (const C2<float>*)s->psi,
+                                       (const float*)s->V, (C2<float>*)s->ya, sh, m,
+                                       s->stream);
+      else if (p.flags & NLSE_FLAG_FMA)
+        e = launch_step1d_fma(s->g, p.method, p.bc, s->cd, (const C2<double>*)s->psi,
+                              (const double*)s->V, (C2<double>*)s->ya, sh, m, s->stream);
+      else
+        e = launch_step1d_exact<double>(s->g, p.method, p.bc, s->cd, (const C2<double>*)s->psi,
+                                        (const double*)s->V, (C2<double>*)s->ya, sh, m,
+                                        s->stream);
+      void* t = s->psi;
+      s->psi = s->ya;
+      s->ya = t;
+      s->flip = 1 - s->flip;
+    }
+    if (e != cudaSuccess) return fail(NLSE_ERR_CUDA, "1D step launch failed: %s", cudaGetErrorString(e));
+    nsteps -= m;
+  }
+  return NLSE_OK;
+}
+
 extern "C" int nlse_solver_run(nlse_solver* s, long long nsteps) {
   if (!s) return fail(NLSE_ERR_ARG, "solver is NULL");
   if (nsteps < 0) return fail(NLSE_ERR_ARG, "nsteps must be >= 0");
   CUDA_TRY(cudaSetDevice(s->device));
+  const Step1dShape sh =
+      step1d_shape(s->g, s->prob.method, s->prob.precision, s->kernel_kind);
+  if (sh.steps) return run_step1d(s, sh, nsteps);
   if (s->g.ndim == 1 && s->g.n <= g_small1d_max && s->prob.precision != NLSE_PREC_DOUBLE &&
       (s->prob.method == 1 || s->dsc) && nsteps > 0)
     return run_small1d(s, nsteps);
@@ -779,7 +818,7 @@ extern "C" int nlse_solver_run(nlse_solver* s, long long nsteps) {
   if (G > 0 && nsteps >= G) {
     long long reps = nsteps / G;
     for (long long t = 0; t < reps; ++t) {
-      int parity = s->prob.precision == NLSE_PREC_MIXED ? s->cur : 0;
+      int parity = s->prob.precision == NLSE_PREC_MIXED ? s->cur : s->flip;
       int r = ensure_graph(s, parity);
       if (r) return r;
       CUDA_TRY(cudaGraphLaunch(s->gexec[parity], s->stream));

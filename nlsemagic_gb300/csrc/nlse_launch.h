@@ -117,6 +117,26 @@ cudaError_t mass_c2f(const C2<float>* psi, long long n, double* out, int* bad, c
 cudaError_t mass_hilo(const float2* hi, const float2* lo, long long n, double* out, int* bad,
                       cudaStream_t st);
 
+// The form a 1D solve's run takes: RK4 steps per launch (0: the stage
+// launches), points per lane, warps per block, launches overlapped (PDL).
+struct Step1dShape {
+  int steps, per_lane, warps;
+  bool pdl;
+};
+Step1dShape step1d_shape(const Geom& g, int method, int precision, int kernel_kind);
+// Whole RK4 steps of a 1D solve in registers (kern_step1d.cuh): m <= sh.steps
+// steps, from one state buffer into another.
+template <typename R>
+cudaError_t launch_step1d_exact(const Geom& g, int method, int BC, const Consts<R>& c,
+                                const C2<R>* in, const R* V, C2<R>* out, const Step1dShape& sh, int m,
+                                cudaStream_t st);
+cudaError_t launch_step1d_fma(const Geom& g, int method, int BC, const Consts<double>& c,
+                              const C2<double>* in, const double* V, C2<double>* out,
+                              const Step1dShape& sh, int m, cudaStream_t st);
+cudaError_t launch_step1d_mixed(const Geom& g, int method, int BC, const Consts<float>& c,
+                                const float2* hi, const float2* lo, const float* V, float2* ho,
+                                float2* l2, const Step1dShape& sh, int m, cudaStream_t st);
+
 bool tiled_supported(const Geom& g, int dim);
 
 // Initial conditions and diagnostics (kern_init.cu); ::nlse_ic is declared
