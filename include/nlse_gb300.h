@@ -185,9 +185,9 @@ int nlse_solver_query(nlse_solver *s, int *idle);
 int nlse_solver_stream(nlse_solver *s, void **stream);
 /* Steps per captured CUDA graph (default 8; 0 disables graphs). */
 int nlse_solver_set_graph_steps(nlse_solver *s, int steps);
-/* Number of kernel launches one RK4 step takes stage by stage.  1D solves
- * run several whole steps per launch where that is faster (knob "seg1d") and
- * then enqueue fewer. */
+/* Number of kernel launches one RK4 step takes stage by stage.  1D and 2D
+ * solves run one or several whole steps per launch where that is faster (knobs
+ * "seg1d", "wide2d.ty") and then enqueue fewer. */
 int nlse_solver_launches_per_step(const nlse_solver *s);
 /* Bytes of device memory held by the solver. */
 long long nlse_solver_device_bytes(const nlse_solver *s);
@@ -303,13 +303,15 @@ int nlse_take_steps_noalloc(const nlse_problem *p, const double *dUr, const doub
  *                  share their halo through L2), 0 every face tile last.
  *                  Same bits either way.
  *   "wide2d"       1 (default): 2D grids (BC 1-3) of the mixed and FP32
- *                  classes take the single-pass stage kernels (one
- *                  launch per stage, the tile staged in shared memory);
- *                  0: the gather kernels (two launches per 2SHOC stage).
- *                  FP32: same bits; mixed: within the mixed tolerance, not
- *                  bit for bit (the single-pass kernel takes the wide form).
- *   "wide2d.ty"    tile height of those kernels: 0 (default) by grid size,
- *                  or 8, 16, 32.  Same bits.
+ *                  classes take the tile kernels (one launch per RK4 step,
+ *                  or one per stage: "wide2d.ty"); 0: the gather kernels
+ *                  (two launches per 2SHOC stage).  FP32: same bits; mixed:
+ *                  within the mixed tolerance, not bit for bit (the tile
+ *                  kernels take the wide form).
+ *   "wide2d.ty"    0 (default): a whole step per launch where that is faster
+ *                  (mixed; FP32 with CD), else a launch per stage with the
+ *                  tile height by grid size; 8, 16 or 32: a launch per stage
+ *                  with that tile height.  Same bits.
  *   "io.zero_copy" 1 (default): host arrays in page-locked memory mapped
  *                  into the device address space (cudaHostAlloc,
  *                  cudaHostRegister) are read and written in place by the

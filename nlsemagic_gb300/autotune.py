@@ -12,8 +12,9 @@ knobs and keeps the fastest:
                    halo re-reads against CTAs in flight),
 * ``graph.steps``  RK4 steps captured per CUDA graph (launch overhead against
                    graph size; matters for small grids),
-* ``wide2d.ty``    tile height of the mixed-precision 2D stage kernel (8, 16
-                   or 32 rows: CTAs in flight against halo re-reads).
+* ``wide2d.ty``    0: a whole step per launch where the library has it for
+                   the grid; 8, 16 or 32: a launch per stage with tiles of
+                   that many rows.
 
 The library has more knobs that give the same bits either way and are not
 tuned here, among them ``wide.pdl`` (1 by default: the 3D 2SHOC stage
@@ -106,7 +107,7 @@ def candidates(shape, precision):
         zcs = [0] + sorted({z for z in (16, 32, 64) if 4 <= z <= L})
         wtys = [4, 8, 16]
     if ndim == 2 and precision == 3:
-        tys = [8, 16, 32]
+        tys = [0, 8, 16, 32]
     for zc in zcs:
         for wty in wtys:
             for ty in tys:

@@ -41,6 +41,8 @@ UNITS = {
     "kern_step1d_exact.cu": ["-fmad=false"],
     "kern_step1d_mixed.cu": [],
     "kern_step1d_fma.cu": [],
+    "kern_step2d_mixed.cu": [],
+    "kern_step2d_exact.cu": ["-fmad=false"],
     "kern_probe.cu": [],
     "kern_exact_fma.cu": [],  # contracted FP64 (NLSE_FLAG_FMA): -fmad left on
     "nlse_batch_fma.cu": [],  # the batched launch's contracted FP64 kernel

@@ -381,7 +381,8 @@ struct nlse_solver {
   int* d_bad;
   // graphs
   int graph_steps;
-  cudaGraphExec_t gexec[2];
+  cudaGraphExec_t gexec[2];  // by the buffer the state is in before (cur, flip)
+  int gflip[2];              // exact classes: the graph leaves it in the other one
   size_t bytes;
 };
 
@@ -647,10 +648,19 @@ extern "C" int nlse_solver_download(nlse_solver* s, double* Ur, double* Ui) {
   return device_error_check();
 }
 
-// Enqueue one RK4 step (4 stage launches) without graphs.
+// Exact classes: the state is now in the other buffer.
+static void flip_state(nlse_solver* s) {
+  void* t = s->psi;
+  s->psi = s->ya;
+  s->ya = t;
+  s->flip = 1 - s->flip;
+}
+
+// Enqueue one RK4 step (4 stage launches, or one step launch) without graphs.
 static int enqueue_step(nlse_solver* s) {
   const nlse_problem& p = s->prob;
   cudaError_t e = cudaSuccess;
+  const int shape = step2d_shape(s->g, p.method, p.bc, p.precision, s->kernel_kind);
   if (p.precision == NLSE_PREC_DOUBLE) {
     typedef C2<double> T;
     T *psi = (T*)s->psi, *K = (T*)s->K, *ya = (T*)s->ya, *yb = (T*)s->yb;
@@ -665,6 +675,10 @@ static int enqueue_step(nlse_solver* s) {
                                        s->kernel_kind)
               : launch_exact_stage<double>(s->g, p.method, p.bc, s->cd, *as[st - 1], st,
                                            s->stream, s->kernel_kind);
+  } else if (shape && p.precision == NLSE_PREC_SINGLE) {
+    e = launch_step2d_exact(s->g, p.bc, s->cf, (const C2<float>*)s->psi, (const float*)s->V,
+                            (C2<float>*)s->ya, shape, s->stream);
+    flip_state(s);
   } else if (p.precision == NLSE_PREC_SINGLE) {
     typedef C2<float> T;
     T *psi = (T*)s->psi, *K = (T*)s->K, *ya = (T*)s->ya, *yb = (T*)s->yb;
@@ -676,6 +690,11 @@ static int enqueue_step(nlse_solver* s) {
     for (int st = 1; st <= 4 && e == cudaSuccess; ++st)
       e = launch_exact_stage<float>(s->g, p.method, p.bc, s->cf, *as[st - 1], st, s->stream,
                                     s->kernel_kind);
+  } else if (shape) {
+    const int c = s->cur;
+    e = launch_step2d_mixed(s->g, p.method, p.bc, s->cf, s->hi[c], s->lo[c], s->Vf, s->mK,
+                            s->hi[1 - c], s->lo[1 - c], shape, s->stream);
+    s->cur = 1 - c;
   } else {
     int c = s->cur;
     float4* G = s->gh;
@@ -715,12 +734,15 @@ static int ensure_graph(nlse_solver* s, int parity) {
   if (s->gexec[parity]) return NLSE_OK;
   cudaGraph_t graph = nullptr;
   int saved_cur = s->cur;
+  const int saved_flip = s->flip;
   s->cur = parity;
   CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   int r = NLSE_OK;
   for (int t = 0; t < s->graph_steps && !r; ++t) r = enqueue_step(s);
   cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
   s->cur = saved_cur;
+  s->gflip[parity] = s->flip != saved_flip;
+  if (s->gflip[parity]) flip_state(s);
   if (r) {
     if (graph) cudaGraphDestroy(graph);
     return r;
@@ -786,10 +808,7 @@ static int run_step1d(nlse_solver* s, const Step1dShape& sh, long long nsteps) {
         e = launch_step1d_exact<double>(s->g, p.method, p.bc, s->cd, (const C2<double>*)s->psi,
                                         (const double*)s->V, (C2<double>*)s->ya, sh, m,
                                         s->stream);
-      void* t = s->psi;
-      s->psi = s->ya;
-      s->ya = t;
-      s->flip = 1 - s->flip;
+      flip_state(s);
     }
     if (e != cudaSuccess) return fail(NLSE_ERR_CUDA, "1D step launch failed: %s", cudaGetErrorString(e));
     nsteps -= m;
@@ -822,7 +841,11 @@ extern "C" int nlse_solver_run(nlse_solver* s, long long nsteps) {
       int r = ensure_graph(s, parity);
       if (r) return r;
       CUDA_TRY(cudaGraphLaunch(s->gexec[parity], s->stream));
-      if (s->prob.precision == NLSE_PREC_MIXED && (G & 1)) s->cur = 1 - s->cur;
+      if (s->prob.precision == NLSE_PREC_MIXED) {
+        if (G & 1) s->cur = 1 - s->cur;
+      } else if (s->gflip[parity]) {
+        flip_state(s);
+      }
     }
     nsteps -= reps * G;
   }

@@ -137,6 +137,16 @@ cudaError_t launch_step1d_mixed(const Geom& g, int method, int BC, const Consts<
                                 const float2* hi, const float2* lo, const float* V, float2* ho,
                                 float2* l2, const Step1dShape& sh, int m, cudaStream_t st);
 
+// Whole RK4 steps of a 2D solve, one launch each (kern_step2d.cuh): the tile
+// shape (0: the stage launches), and one step from one state buffer pair into
+// the other.
+int step2d_shape(const Geom& g, int method, int BC, int precision, int kernel_kind);
+cudaError_t launch_step2d_mixed(const Geom& g, int method, int BC, const Consts<float>& c,
+                                const float2* hi, const float2* lo, const float* V, float2* K,
+                                float2* ho, float2* l2, int shape, cudaStream_t st);
+cudaError_t launch_step2d_exact(const Geom& g, int BC, const Consts<float>& c, const C2<float>* in,
+                                const float* V, C2<float>* out, int shape, cudaStream_t st);
+
 bool tiled_supported(const Geom& g, int dim);
 
 // Initial conditions and diagnostics (kern_init.cu); ::nlse_ic is declared

@@ -198,18 +198,18 @@ __device__ __forceinline__ float2 f_boundary(const Consts<float>& c, const HE& u
 }
 
 // ---- compensated update psi += inc, psi = (hi, lo) -------------------------
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& t) {
-  s = __fadd_rn(a, b);
-  float bb = __fsub_rn(s, a);
-  t = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+__device__ __forceinline__ void two_sum(float2 a, float2 b, float2& s, float2& t) {
+  s = padd(a, b);
+  const float2 bb = psub(s, a);
+  t = padd(psub(a, psub(s, bb)), psub(b, bb));
 }
 
-__device__ __forceinline__ void comp_add(float& hi, float& lo, float inc) {
-  float s, t;
+__device__ __forceinline__ void comp_add(float2& hi, float2& lo, float2 inc) {
+  float2 s, t;
   two_sum(hi, inc, s, t);
-  t = __fadd_rn(t, lo);
-  hi = __fadd_rn(s, t);
-  lo = __fsub_rn(t, __fsub_rn(hi, s));
+  t = padd(t, lo);
+  hi = padd(s, t);
+  lo = psub(t, psub(hi, s));
 }
 
 // ---- RK4 stage update of the mixed path -------------------------------------
@@ -251,8 +251,7 @@ __device__ __forceinline__ void stage_update(const Consts<float>& c, int stage, 
     const float2 inc = pfma(P2(0x1.555556p-2f), y, pmul(P2(-0x1.555556p-27f), y));
     hio = hi;
     loo = lo;
-    comp_add(hio.x, loo.x, inc.x);
-    comp_add(hio.y, loo.y, inc.y);
+    comp_add(hio, loo, inc);
   }
 }
 
