@@ -276,6 +276,10 @@ int nlse_take_steps_noalloc(const nlse_problem *p, const double *dUr, const doub
  *   "wide.zc"      z-chunk length of the mixed-precision 3D kernel (planes a
  *                  CTA streams through); 0 = built-in heuristic.
  *   "graph.steps"  RK4 steps per captured graph for new solvers (default 8).
+ *   The wide.* knobs choose between forms of the mixed-precision 3D streaming
+ *   kernels.  Small 3D grids, and grids with an odd number of points a row,
+ *   run by point instead (one launch per stage, same bits) while "wide.pdl",
+ *   "wide.strips", "wide.z2" and "wide.tile_order" are all 1.
  *   "wide.pdl"     1 (default): the mixed-precision 3D 2SHOC stage kernels
  *                  (face ghosts, interior, faces) are launched with
  *                  programmatic dependent launch, so a stage's interior

@@ -41,6 +41,9 @@ from . import _lib
 from .api import Solver, grid_dims
 
 KNOBS = ("wide.zc", "wide.ty", "graph.steps", "wide2d.ty")
+# the library's own choice, timed beside the candidates (2D: a whole step per
+# launch, which no tile height of the stage kernels selects)
+DEFAULTS = {"wide.zc": 0, "wide.ty": 8, "graph.steps": 8, "wide2d.ty": 0}
 
 
 def set_knob(key, value):
@@ -107,7 +110,7 @@ def candidates(shape, precision):
         zcs = [0] + sorted({z for z in (16, 32, 64) if 4 <= z <= L})
         wtys = [4, 8, 16]
     if ndim == 2 and precision == 3:
-        tys = [0, 8, 16, 32]
+        tys = [8, 16, 32]
     for zc in zcs:
         for wty in wtys:
             for ty in tys:
@@ -165,7 +168,7 @@ def tune(shape, method=2, precision=3, BC=2, steps=20, force=False, verbose=Fals
     results = []
     sv = _solver_for(shape, method, precision, BC)
     try:
-        for cfg in candidates(shape, precision):
+        for cfg in [dict(DEFAULTS)] + candidates(shape, precision):
             t = time_config(shape, method, precision, BC, cfg, steps, solver=sv)
             results.append((t, cfg))
             if verbose:

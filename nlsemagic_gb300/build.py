@@ -45,6 +45,9 @@ UNITS = {
     "kern_step2d_exact.cu": ["-fmad=false"],
     "kern_probe.cu": [],
     "kern_exact_fma.cu": [],  # contracted FP64 (NLSE_FLAG_FMA): -fmad left on
+    "kern_point_fma.cu": [],
+    "kern_point_mixed.cu": [],
+    "kern_point_exact.cu": ["-fmad=false"],
     "nlse_batch_fma.cu": [],  # the batched launch's contracted FP64 kernel
 }
 

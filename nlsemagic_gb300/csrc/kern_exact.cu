@@ -10,19 +10,42 @@ static bool tile2d_path(const Geom& g, int method, int BC, int kernel_kind, bool
   return g.ndim == 2 && single && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_wide2d;
 }
 
-// D scratch: 2SHOC in gather form.  FP32 2D grids on the tile kernel take
-// none; should the knob turn it off later, the gather kernel recomputes D.
+// Thread-per-point stages (kern_point.cuh).  FP64 takes them in 2D and 3D: its
+// issue rate is the bound, and they waste least of it.  Microseconds a step of
+// one solve alone / of three in flight, against the gather kernels (2D) and the
+// tiled ones (3D), MSD:
+//   CD     200^2 40.3 / 24.9 -> 25.6 / 13.2    1500^2 514 / 485 -> 480 / 469
+//          61 x 72 x 67 185 / 137 -> 101 / 70  200^3 2743 / 2419 -> 1912 / 1896
+//   2SHOC  200^2 108 / 43.5 -> 48.5 / 25.4     1500^2 1001 / 952 -> 930 / 912
+//          61 x 72 x 67 546 / 386 -> 257 / 171 200^3 8221 / 7653 -> 4692 / 4660
+// FP32 is bound by L1 there.  2SHOC in 3D gains all the same, D no longer formed
+// on a tile's halo (61 x 72 x 67 124 / 62 -> 42 / 26, 220^3 1294 / 1143 -> 768 /
+// 757, Dirichlet 919 / 762 -> 771 / 758); CD, which the tiled kernel streams
+// through once, up to 2^20 points (96^3 52 / 32 -> 35 / 32), where the state's
+// rows do not start on 16 bytes and TMA cannot stage them (161 x 150 x 155 274 /
+// 248 -> 127 / 123), and with MSD (160^3 186 / 145 -> 147 / 140; Dirichlet 168 /
+// 131 against 146 / 140 stays tiled).
+static bool point_path(const Geom& g, int method, int BC, int kernel_kind, bool single) {
+  if (kernel_kind != KERNEL_TILED || BC > 3) return false;
+  if (!single) return g.ndim >= 2;
+  return g.ndim == 3 && (method == 2 || BC == 2 || g.M % 2 || g.n <= (1LL << 20));
+}
+
+// D scratch: 2SHOC in gather form and by point.  FP32 2D grids on the tile
+// kernel take none; should the knob turn it off later, the gather kernel
+// recomputes D.
 long long exact_dsc_entries(const Geom& g, int method, int BC, int kernel_kind, bool single) {
   if (method != 2) return 0;
-  const bool tiled = kernel_kind == KERNEL_TILED && tiled_supported(g, g.ndim) && BC != 4;
-  return tiled || tile2d_path(g, method, BC, kernel_kind, single) ? 0 : g.n;
+  return tile2d_path(g, method, BC, kernel_kind, single) ? 0 : g.n;
 }
 
 int exact_stage_launches(const Geom& g, int method, int BC, int kernel_kind, bool single,
                          bool has_dsc) {
   if (tile2d_path(g, method, BC, kernel_kind, single)) return 1;
   if (seg1d_exact_path(g, method, BC, kernel_kind, single)) return 1;
-  if (kernel_kind == KERNEL_TILED && tiled_supported(g, g.ndim) && BC != 4) return 1;
+  if (kernel_kind == KERNEL_TILED && tiled_supported(g, g.ndim) && BC != 4 &&
+      !point_path(g, method, BC, kernel_kind, single))
+    return 1;
   return method == 2 && has_dsc ? 2 : 1;  // (D,) F
 }
 
@@ -30,6 +53,9 @@ template <typename R>
 cudaError_t launch_exact_stage(const Geom& g, int method, int BC, const Consts<R>& c,
                                const ExactStageArgs<R>& a, int stage, cudaStream_t st,
                                int kernel_kind) {
+  // (the allocation-free call has no D scratch: its 2SHOC forms D on the way)
+  if (point_path(g, method, BC, kernel_kind, sizeof(R) == 4) && (method == 1 || a.dsc))
+    return launch_point_exact<R>(g, method, BC, c, a, stage, st);
   return launch_exact_stage_var<R, 0>(g, method, BC, c, a, stage, st, kernel_kind);
 }
 

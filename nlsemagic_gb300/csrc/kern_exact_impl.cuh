@@ -25,8 +25,11 @@ inline bool seg1d_exact_path(const Geom& g, int method, int BC, int kernel_kind,
 template <typename R, int DIM, int METHOD, int BC, int VAR>
 cudaError_t launch_one(const Geom& g, const Consts<R>& c, const ExactStageArgs<R>& a,
                               int stage, cudaStream_t st, int kernel_kind) {
-  if (kernel_kind == KERNEL_TILED && tiled_supported(g, DIM)) {
-    return tiled::launch_exact<R, DIM, METHOD, BC, VAR>(g, c, a, stage, st);
+  // 3D, what does not go by point (kern_exact.cu): FP32 with CD, and FP64
+  // 2SHOC without D scratch
+  if constexpr (VAR == 0 && DIM == 3 && BC != 4 && (sizeof(R) == 4) == (METHOD == 1)) {
+    if (kernel_kind == KERNEL_TILED && tiled_supported(g, DIM))
+      return tiled::launch_exact<R, DIM, METHOD, BC>(g, c, a, stage, st);
   }
   // FP64 1D grids above the step kernel's limit (kern_step1d.cuh): staged
   // segments, one launch per stage, below 2^22 points (bound by FP64 issue,

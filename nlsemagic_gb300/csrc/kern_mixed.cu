@@ -77,8 +77,24 @@ static bool wide_path(const Geom& g, int BC, int kernel_kind) {
   return kernel_kind == KERNEL_TILED && g.ndim == 3 && tiled_supported(g, 3) && BC != 4;
 }
 
+// 3D stages by point (kern_point_mixed.cu): small grids, and grids whose rows
+// do not start on 16 bytes, which the streaming kernels stage without TMA.
+// Microseconds a step of one solve alone / of three in flight, MSD, streaming ->
+// by point: 2SHOC 32^3 99 / 35 -> 29 / 12, 61 x 72 x 67 139 / 52 -> 27 / 17, 80^3
+// 112 / 47 -> 37 / 35, 128 x 100 x 81 126 / 81 -> 65 / 80, 128^3 151 / 128 against
+// 154 / 162, 161 x 150 x 155 356 / 289 -> 285 / 279; CD 61 x 72 x 67 87 / 33 ->
+// 21 / 11, 80^3 53 / 27 -> 26 / 19, 96^3 Dirichlet 50 / 31 against 34 / 34, 161 x
+// 150 x 155 283 / 235 -> 159 / 155.  The knobs that choose between forms of the
+// streaming kernels choose those kernels; grids 3 cells thin, all face, stay
+// with them too.
+bool mixed_point_path(const Geom& g, int method, int BC, int kernel_kind) {
+  if (!wide_path(g, BC, kernel_kind) || g.M < 4 || g.N < 4 || g.L < 4) return false;
+  if (!wide::g_pdl || !wide::g_strips || !wide::g_z2 || !wide::g_tile_order) return false;
+  return g.M % 2 || g.n <= (method == 1 ? 3LL << 18 : 1LL << 20);
+}
+
 bool mixed_strip_path(const Geom& g, int method, int BC, int kernel_kind) {
-  return wide::g_strips && method == 2 && wide_path(g, BC, kernel_kind);
+  return !mixed_point_path(g, method, BC, kernel_kind) && wide::g_strips && method == 2 && wide_path(g, BC, kernel_kind);
 }
 
 // x-face strips of lo and V, and V next to the faces, from the full arrays
@@ -109,6 +125,7 @@ cudaError_t mixed_strip_fill(const Geom& g, const float2* lo, const float* V, fl
 int mixed_stage_launches(const Geom& g, int method, int BC, int kernel_kind, bool has_dsc) {
   if (g.ndim == 2 && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_wide2d) return 1;
   if (g.ndim == 1 && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_seg1d) return 1;
+  if (mixed_point_path(g, method, BC, kernel_kind)) return 1;
   if (!wide_path(g, BC, kernel_kind)) return method == 2 && has_dsc ? 2 : 1;  // (D,) F
   return method == 2 ? 3 : 2;  // (ghosts,) interior, faces
 }
@@ -135,6 +152,8 @@ long long mixed_fq_entries(const Geom& g, int method, int BC, int kernel_kind) {
 cudaError_t launch_mixed_stage(const Geom& g, int method, int BC, const Consts<float>& c,
                                const MixedStageArgs& a, int stage, cudaStream_t st,
                                int kernel_kind) {
+  if (mixed_point_path(g, method, BC, kernel_kind))
+    return launch_point_mixed(g, method, BC, c, a, stage, st);
   if (method == 1) {
     switch (g.ndim) {
       case 1: return by_bc<1, 1>(g, BC, c, a, stage, st, kernel_kind);

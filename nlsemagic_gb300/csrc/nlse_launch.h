@@ -19,7 +19,7 @@ struct ExactStageArgs {
   const R* V;
   C2<R>* K;
   C2<R>* Yout;       // next stage input (stages 1-3)
-  C2<R>* dsc;        // 2SHOC on the gather path: D scratch (n points), or null
+  C2<R>* dsc;        // 2SHOC by gather or by point: D scratch (n points), or null
 };
 
 struct MixedStageArgs {
@@ -66,6 +66,17 @@ cudaError_t launch_exact_stage_fma(const Geom& g, int method, int BC, const Cons
                                    const ExactStageArgs<double>& a, int stage, cudaStream_t st,
                                    int kernel_kind);
 
+// Thread-per-point stages in 2D and 3D (kern_point.cuh): exact, contracted.
+template <typename R>
+cudaError_t launch_point_exact(const Geom& g, int method, int BC, const Consts<R>& c,
+                               const ExactStageArgs<R>& a, int stage, cudaStream_t st);
+cudaError_t launch_point_fma(const Geom& g, int method, int BC, const Consts<double>& c,
+                             const ExactStageArgs<double>& a, int stage, cudaStream_t st);
+// 3D, mixed (kern_point_mixed.cu), and which grids take it.
+bool mixed_point_path(const Geom& g, int method, int BC, int kernel_kind);
+cudaError_t launch_point_mixed(const Geom& g, int method, int BC, const Consts<float>& c,
+                               const MixedStageArgs& a, int stage, cudaStream_t st);
+
 cudaError_t launch_mixed_stage(const Geom& g, int method, int BC, const Consts<float>& c,
                                const MixedStageArgs& a, int stage, cudaStream_t st,
                                int kernel_kind);
@@ -89,8 +100,8 @@ int exact_stage_launches(const Geom& g, int method, int BC, int kernel_kind, boo
                          bool has_dsc);
 long long mixed_ghost_entries(const Geom& g, int method, int BC, int kernel_kind);
 long long mixed_fq_entries(const Geom& g, int method, int BC, int kernel_kind);
-// Points of D scratch (ExactStageArgs / MixedStageArgs ::dsc) a 2SHOC stage on
-// the gather path uses (two launches per stage), else 0.
+// Points of D scratch (ExactStageArgs / MixedStageArgs ::dsc) a 2SHOC stage
+// uses that takes two launches, else 0.
 long long exact_dsc_entries(const Geom& g, int method, int BC, int kernel_kind, bool single);
 long long mixed_dsc_entries(const Geom& g, int method, int BC, int kernel_kind);
 
