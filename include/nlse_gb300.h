@@ -199,9 +199,11 @@ long long nlse_solver_bytes_for(const nlse_problem *p);
 /* ------------------------------------------------------------------------
  * Batched solves: many independent solves of uneven dimension, size,
  * method, boundary code and precision class (FP64 or mixed) advance together
- * in one persistent cooperative launch per call of nlse_batch_run, driven by
- * a tile work queue (one pass over all tiles per RK4 stage, separated by a
- * bounded grid barrier).  State lives in a device pool of a fixed byte
+ * in one persistent launch per precision class and call of nlse_batch_run,
+ * driven by a tile work queue: mixed 1D and 2D solves in whole RK4 steps
+ * ordered per solve; everything else (and a run whose mixed solves include a
+ * 3D one) one pass over all tiles per RK4 stage, separated by a bounded grid
+ * barrier.  State lives in a device pool of a fixed byte
  * budget; solves are admitted while the pool has room and keep their state
  * resident until removed.  No reference counterpart (the reference runs one
  * solve per MEX call).
@@ -236,7 +238,8 @@ int nlse_batch_query(nlse_batch *b, int *idle);
 int nlse_batch_stats(nlse_batch *b, int *active, long long *points, long long *free_bytes);
 /* cudaStream_t of the batch. */
 int nlse_batch_stream(nlse_batch *b, void **stream);
-/* Kernel launches issued by the last nlse_batch_run (1 when any solve ran). */
+/* Kernel launches issued by the last nlse_batch_run (one per
+ * precision class that ran). */
 int nlse_batch_last_launches(nlse_batch *b);
 
 /* ------------------------------------------------------------------------

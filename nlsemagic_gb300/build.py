@@ -48,6 +48,7 @@ UNITS = {
     "kern_point_fma.cu": [],
     "kern_point_mixed.cu": [],
     "kern_point_exact.cu": ["-fmad=false"],
+    "nlse_batch_steps.cu": [],
     "nlse_batch_fma.cu": [],  # the batched launch's contracted FP64 kernel
 }
 

@@ -46,7 +46,7 @@ struct Plan {
 };
 
 // Windows of m steps over n points, R per lane.
-inline Plan make_plan(long long n, int method, int R, int m, int warps) {
+__host__ __device__ inline Plan make_plan(long long n, int method, int R, int m, int warps) {
   Plan p;
   p.m = m;
   p.lost = n <= 32 * R ? 0 : 4 * (method == 2 ? 2 : 1) * m;
@@ -122,19 +122,16 @@ __device__ __forceinline__ void put(T (&a)[R], int pos, int lane, T v) {
 // ---- mixed class --------------------------------------------------------------
 // The hi parts do not change within a step: their share of the Laplacian,
 // (h+ - h0) + (h- - h0), is formed once per step (mixed::lapsum, split).
+// One window, by the calling warp; first: the first point it stores.
 template <int METHOD, int BC, int R>
-__global__ void __launch_bounds__(32 * MAX_WARPS)
-    mixed_steps(int n, Consts<float> c, const float2* hi_in, const float2* lo_in, const float* V,
-                float2* hi_out, float2* lo_out, Plan pl) {
+__device__ __forceinline__ void mixed_window(int n, const Consts<float>& c, const float2* hi_in,
+                                             const float2* lo_in, const float* V, float2* hi_out,
+                                             float2* lo_out, const Plan& pl, int first) {
   using namespace mixed;
   constexpr int W = 32 * R;
-  pdl_trigger();  // the next kernel may launch; it waits for this one
   const int lane = (int)(threadIdx.x & 31);
-  const int first = (int)(blockIdx.x * pl.warps + (threadIdx.x >> 5)) * pl.U;
-  if (first >= n) return;
   const int x0 = first - pl.lost, x = x0 + lane * R;
   const bool ends = x0 <= 0 || x0 + W >= n;  // an end of the grid in the window
-  pdl_wait();  // the previous kernel's output
   float2 hi[R], lo[R], e[R], sh[R], K[R], T[R];
   float v[R];
 #pragma unroll
@@ -232,6 +229,17 @@ __global__ void __launch_bounds__(32 * MAX_WARPS)
       lo_out[x + r] = lo[r];
     }
   }
+}
+
+template <int METHOD, int BC, int R>
+__global__ void __launch_bounds__(32 * MAX_WARPS)
+    mixed_steps(int n, Consts<float> c, const float2* hi_in, const float2* lo_in, const float* V,
+                float2* hi_out, float2* lo_out, Plan pl) {
+  pdl_trigger();  // the next kernel may launch; it waits for this one
+  const int first = (int)(blockIdx.x * pl.warps + (threadIdx.x >> 5)) * pl.U;
+  if (first >= n) return;
+  pdl_wait();  // the previous kernel's output
+  mixed_window<METHOD, BC, R>(n, c, hi_in, lo_in, V, hi_out, lo_out, pl, first);
 }
 
 // ---- exact classes (FP64 / FP32) ---------------------------------------------

@@ -53,12 +53,12 @@ struct Tile {
 };
 
 template <int H>
-__device__ __forceinline__ Tile tile_of(const Geom& g, int nbx, int nby) {
+__device__ __forceinline__ Tile tile_of(const Geom& g, int bx, int by, int nbx, int nby) {
   Tile t;
-  t.tx0 = (int)((long long)blockIdx.x * g.M / nbx);
-  t.tx1 = (int)((long long)(blockIdx.x + 1) * g.M / nbx);
-  t.ty0 = (int)((long long)blockIdx.y * g.N / nby);
-  t.ty1 = (int)((long long)(blockIdx.y + 1) * g.N / nby);
+  t.tx0 = (int)((long long)bx * g.M / nbx);
+  t.tx1 = (int)((long long)(bx + 1) * g.M / nbx);
+  t.ty0 = (int)((long long)by * g.N / nby);
+  t.ty1 = (int)((long long)(by + 1) * g.N / nby);
   t.x0 = t.tx0 - 3 * H;
   t.y0 = t.ty0 - 3 * H;
   return t;
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(XT* G, MINB)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* const sm = reinterpret_cast<float2*>(smem_raw);
   pdl_trigger();  // the next kernel may launch; it waits for this one
-  const Tile t = tile_of<H>(g, nbx, nby);
+  const Tile t = tile_of<H>(g, (int)blockIdx.x, (int)blockIdx.y, nbx, nby);
   pdl_wait();  // the previous kernel's output
   if (at_edge<H>(g, t))
     mixed_tile<METHOD, BC, XT, G, R, true>(g, c, hi_in, lo_in, V, Kg, hi_out, lo_out, t, sm);

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(XT* G, MINB)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C2<float>* const sm = reinterpret_cast<C2<float>*>(smem_raw);
   pdl_trigger();  // the next kernel may launch; it waits for this one
-  const Tile t = tile_of<1>(g, nbx, nby);
+  const Tile t = tile_of<1>(g, (int)blockIdx.x, (int)blockIdx.y, nbx, nby);
   pdl_wait();  // the previous kernel's output
   if (at_edge<1>(g, t))
     exact_cd_tile<BC, XT, G, R, true>(g, c, in, V, out, t, sm);

@@ -1,11 +1,13 @@
 // Batched solves in one persistent launch (C ABI: nlse_batch_* in
 // include/nlse_gb300.h).
 //
-// Device side (batch_kern.cuh): a cooperative persistent kernel.  All active solves are cut
+// Device side: a run whose mixed solves are all 1D or 2D takes them in whole RK4
+// steps (nlse_batch_steps.cu).  Everything else (batch_kern.cuh): a cooperative
+// persistent kernel.  All active solves are cut
 // into tiles; per RK4 stage every CTA pulls tiles from an atomic work-queue
 // counter of that stage until the queue is empty, evaluates the stage on the
 // tile, and then waits at a grid barrier.  Tiles by solve:
-//   - mixed 2D (BC 1-3): 32 x 16 rectangles, the single-pass 2D stage tile
+//   - mixed 2D (BC 1-3): 32 x 32 rectangles, the single-pass 2D stage tile
 //     (kern_wide2d.cuh: same bits as the single-solve 2D kernel);
 //   - mixed 1D (BC 1-3): segments of 1024 points staged in shared memory,
 //     D formed there (kern_seg1d.cuh: same bits as the gather kernels);
@@ -34,9 +36,17 @@
 #include "batch_kern.cuh"
 
 // Shared with nlse_abi.cu: error reporting, validation, scalar constants;
-// from nlse_batch_fma.cu: the contracted FP64 kernel.
+// from nlse_batch_steps.cu: the kernel for mixed 1D and 2D solves; from
+// nlse_batch_fma.cu: the contracted FP64 kernel.
 namespace nlse {
 int set_error(int code, const char* fmt, ...);
+bool batch_steps_takes(const nlse_problem& p);
+long long batch_steps_tiles(const void* solve);
+long long batch_steps_rounds(const void* solve, long long adv);
+cudaError_t batch_steps_launch(const void* solves, const void* tiles, int ntiles,
+                               const int* tile_n, int max_steps, long long rounds,
+                               unsigned long long* queue, int* err, long long budget, int sms,
+                               cudaStream_t st);
 int batch_fma_blocks_per_sm();
 cudaError_t batch_fma_launch(unsigned blocks, void** args, cudaStream_t st);
 }
@@ -84,8 +94,13 @@ struct nlse_batch {
   // staging for transfers (planar doubles)
   double* stage = nullptr;
   size_t stage_cap = 0;
-  // resident CTAs: FP64, mixed, mixed with staged tiles only, contracted FP64
-  int max_blocks[4] = {0, 0, 0, 0};
+  // step launch (nlse_batch_steps.cu): task and per-solve counters, tiles a
+  // round per solve (device, pinned host)
+  unsigned long long* d_queue = nullptr;
+  int *d_tile_n = nullptr, *h_tile_n = nullptr;
+  int sms = 0;
+  // resident CTAs: FP64, mixed, contracted FP64
+  int max_blocks[3] = {0, 0, 0};
   int last_launches = 0;
 };
 
@@ -153,11 +168,13 @@ extern "C" int nlse_batch_destroy(nlse_batch* b) {
   if (!b) return NLSE_OK;
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
-  void* dp[] = {b->pool, b->d_solves, b->d_tiles, b->d_qctr, b->d_bar, b->d_err, b->stage};
+  void* dp[] = {b->pool, b->d_solves, b->d_tiles, b->d_qctr, b->d_bar, b->d_err, b->stage,
+                b->d_queue, b->d_tile_n};
   for (void* p : dp)
     if (p) cudaFree(p);
   if (b->h_solves) cudaFreeHost(b->h_solves);
   if (b->h_tiles) cudaFreeHost(b->h_tiles);
+  if (b->h_tile_n) cudaFreeHost(b->h_tile_n);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
   return NLSE_OK;
@@ -185,27 +202,25 @@ extern "C" int nlse_batch_create(long long pool_bytes, int max_solves, nlse_batc
   if (cudaMalloc(&b->d_solves, sizeof(BSolve) * max_solves) != cudaSuccess ||
       cudaMalloc(&b->d_bar, sizeof(BarrierState)) != cudaSuccess ||
       cudaMalloc(&b->d_err, sizeof(int)) != cudaSuccess ||
+      cudaMalloc(&b->d_queue, sizeof(unsigned long long) * (max_solves + 1)) != cudaSuccess ||
+      cudaMalloc(&b->d_tile_n, sizeof(int) * max_solves) != cudaSuccess ||
+      cudaMallocHost(&b->h_tile_n, sizeof(int) * max_solves) != cudaSuccess ||
       cudaMallocHost(&b->h_solves, sizeof(BSolve) * max_solves) != cudaSuccess) {
     cudaGetLastError();
     return cleanup(nlse::set_error(NLSE_ERR_NOMEM, "batch table allocation failed"));
   }
   cudaMemsetAsync(b->d_bar, 0, sizeof(BarrierState), b->stream);
   cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream);
-  int sms = 0, per64 = 0, permx = 0, perst = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per64, batch_kernel<NLSE_PREC_DOUBLE, false>,
-                                                BT, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&permx, batch_kernel<NLSE_PREC_MIXED, false>,
-                                                BT, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perst, batch_kernel<NLSE_PREC_MIXED, true>,
-                                                BT, 0);
+  int per64 = 0, permx = 0;
+  cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per64, batch_kernel<NLSE_PREC_DOUBLE>, BT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&permx, batch_kernel<NLSE_PREC_MIXED>, BT, 0);
   const int perfma = nlse::batch_fma_blocks_per_sm();
-  if (per64 < 1 || permx < 1 || perst < 1 || perfma < 1)
+  if (per64 < 1 || permx < 1 || perfma < 1)
     return cleanup(nlse::set_error(NLSE_ERR_CUDA, "batch kernel cannot be resident"));
-  b->max_blocks[0] = sms * per64;
-  b->max_blocks[1] = sms * permx;
-  b->max_blocks[2] = sms * perst;
-  b->max_blocks[3] = sms * perfma;
+  b->max_blocks[0] = b->sms * per64;
+  b->max_blocks[1] = b->sms * permx;
+  b->max_blocks[2] = b->sms * perfma;
   *out = b;
   return NLSE_OK;
 }
@@ -312,6 +327,15 @@ extern "C" int nlse_batch_run(nlse_batch* b, int max_steps) {
   std::vector<int> which[NC];
   long long ntiles[NC] = {0, 0, 0}, ntiles_d[NC] = {0, 0, 0};
   int steps[NC] = {0, 0, 0};
+  // mixed 1D and 2D solves alone: whole steps per task (nlse_batch_steps.cu)
+  bool stepwise = true;
+  for (const Slot& S : b->slots)
+    if (S.used && S.d.steps_left > 0 && S.d.prec != NLSE_PREC_DOUBLE)
+      stepwise = stepwise && nlse::batch_steps_takes(S.prob);
+  auto count = [&](const BSolve& d) {
+    return stepwise && d.prec != NLSE_PREC_DOUBLE ? nlse::batch_steps_tiles(&d) : tile_count(d);
+  };
+  long long rounds = 0;  // of the step launch
   for (int pass = 0; pass < 2; ++pass)  // D-phase solves, then the others
     for (size_t t = 0; t < b->slots.size(); ++t) {
       Slot& S = b->slots[t];
@@ -319,10 +343,14 @@ extern "C" int nlse_batch_run(nlse_batch* b, int max_steps) {
       if (!S.used || S.d.steps_left <= 0 || dphase != (pass == 0)) continue;
       const int c = S.d.prec != NLSE_PREC_DOUBLE ? 1 : (S.prob.flags & NLSE_FLAG_FMA) ? 2 : 0;
       which[c].push_back((int)t);
-      const long long nt = tile_count(S.d);
+      const long long nt = count(S.d);
       ntiles[c] += nt;
       if (pass == 0) ntiles_d[c] += nt;
       long long adv = S.d.steps_left < max_steps ? S.d.steps_left : max_steps;
+      if (c == 1 && stepwise) {
+        const long long r = nlse::batch_steps_rounds(&S.d, adv);
+        if (r > rounds) rounds = r;
+      }
       if (adv > steps[c]) steps[c] = (int)adv;
     }
   const long long total_tiles = ntiles[0] + ntiles[1] + ntiles[2];
@@ -355,11 +383,12 @@ extern "C" int nlse_batch_run(nlse_batch* b, int max_steps) {
       Slot& S = b->slots[id];
       b->h_solves[nsolves] = S.d;
       const int kind = tile_kind(S.d);
-      const long long nt = tile_count(S.d);
+      const long long nt = count(S.d);
+      b->h_tile_n[nsolves] = (int)nt;
       for (long long q = 0; q < nt; ++q) {
         b->h_tiles[tt].solve = nsolves;
         b->h_tiles[tt].kind = kind;
-        b->h_tiles[tt].start = kind == K_LINEAR ? q * TILE : q;
+        b->h_tiles[tt].start = kind == K_LINEAR && !(c == 1 && stepwise) ? q * TILE : q;
         ++tt;
       }
       ++nsolves;
@@ -375,12 +404,21 @@ extern "C" int nlse_batch_run(nlse_batch* b, int max_steps) {
       first += ntiles[c];
       continue;
     }
+    if (c == 1 && stepwise) {
+      BTRY(cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned long long) * (nsolves + 1), b->stream));
+      BTRY(cudaMemcpyAsync(b->d_tile_n, b->h_tile_n, sizeof(int) * nsolves,
+                           cudaMemcpyHostToDevice, b->stream));
+      BTRY(nlse::batch_steps_launch(b->d_solves, b->d_tiles + first, (int)ntiles[c], b->d_tile_n,
+                                    steps[c], rounds, b->d_queue, b->d_err, budget, b->sms,
+                                    b->stream));
+      ++b->last_launches;
+      first += ntiles[c];
+      continue;
+    }
     const size_t np = (size_t)steps[c] * 8;
     BTRY(cudaMemsetAsync(b->d_qctr, 0, sizeof(unsigned) * np, b->stream));
     BTRY(cudaMemsetAsync(b->d_bar, 0, sizeof(BarrierState), b->stream));
-    bool staged = c == 1;  // every solve of the class in segment / rectangle tiles
-    for (int id : which[c]) staged = staged && tile_kind(b->slots[id].d) != K_LINEAR;
-    int blocks = b->max_blocks[c == 2 ? 3 : staged ? 2 : c];
+    int blocks = b->max_blocks[c];
     if ((long long)blocks > ntiles[c]) blocks = (int)ntiles[c];
     const BTile* tiles = b->d_tiles + first;
     int nt_i = (int)ntiles[c], ntd_i = (int)ntiles_d[c], st_i = steps[c];
@@ -389,9 +427,8 @@ extern "C" int nlse_batch_run(nlse_batch* b, int max_steps) {
     if (c == 2) {
       BTRY(nlse::batch_fma_launch((unsigned)blocks, args, b->stream));
     } else {
-      const void* kern = c == 0   ? (const void*)batch_kernel<NLSE_PREC_DOUBLE, false>
-                         : staged ? (const void*)batch_kernel<NLSE_PREC_MIXED, true>
-                                  : (const void*)batch_kernel<NLSE_PREC_MIXED, false>;
+      const void* kern = c == 0 ? (const void*)batch_kernel<NLSE_PREC_DOUBLE>
+                                : (const void*)batch_kernel<NLSE_PREC_MIXED>;
       BTRY(cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(BT), args, 0, b->stream));
     }
     ++b->last_launches;
@@ -403,7 +440,9 @@ extern "C" int nlse_batch_run(nlse_batch* b, int max_steps) {
       Slot& S = b->slots[id];
       long long adv = S.d.steps_left < steps[c] ? S.d.steps_left : steps[c];
       S.d.steps_left -= adv;
-      if (S.d.prec == NLSE_PREC_MIXED && (adv & 1)) S.d.cur ^= 1;
+      // the state's buffer: changes every step, or every round of the step launch
+      const long long turns = c == 1 && stepwise ? nlse::batch_steps_rounds(&S.d, adv) : adv;
+      if (S.d.prec == NLSE_PREC_MIXED && (turns & 1)) S.d.cur ^= 1;
     }
   return NLSE_OK;
 }
