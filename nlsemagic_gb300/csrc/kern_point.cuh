@@ -160,14 +160,18 @@ __device__ __forceinline__ C2<R> interior(const Geom& g, const Consts<R>& c, con
   return exact::f_2shoc_3d<R>(c, u[0], v, d[0], dn, e);
 }
 
-// One launch of a stage.  FORM D writes Ds and reads Yin and V only.  VAR: as
+// One launch of a stage.  The deep points trigger the next launch once F is
+// formed, not at the start: its blocks are then placed as this launch ends, which
+// hides its latency.  Placed at the start, while this launch's blocks still come
+// and go, they load the SMs unevenly (FP64 2SHOC on 200 x 333, one solve: 110 us a
+// step; 49 without overlap, 47 so; with three in flight 37, 31 and 30).
+// FORM D writes Ds and reads Yin and V only.  VAR: as
 // exact::gather_stage (1: the contracted class).
 template <typename R, int DIM, Form FORM, int BC, int VAR, int NT>
 __global__ void __launch_bounds__(NT)
     pass(Geom g, Consts<R> c, const C2<R>* Yin, C2<R>* Psi, const R* V, C2<R>* K, C2<R>* Yout,
          C2<R>* Ds, int stage, Map m) {
   typedef C2<R> T2;
-  pdl_trigger();  // the next kernel may launch; it waits for this one
   const int M = g.M, P = g.P;
   if (blockIdx.x >= m.shell_blocks) {
     const unsigned d = (blockIdx.x - m.shell_blocks) * NT + threadIdx.x;
@@ -184,11 +188,17 @@ __global__ void __launch_bounds__(NT)
         t1 = add(t1, axpy(add(u[P], u[-P]), (R)-2, y0));
         s2 = add(s2, add(u[2 * P], u[-2 * P]));
       }
-      exact::update<R>(c, stage, p, rhs_wide<R, DIM>(c, y0, V[p], t1, s2), Psi, K, Yout);
+      const T2 f0 = rhs_wide<R, DIM>(c, y0, V[p], t1, s2);
+      pdl_trigger();
+      exact::update<R>(c, stage, p, f0, Psi, K, Yout);
     } else if (FORM == D) {
-      Ds[p] = interior<R, DIM, D>(g, c, u, (R)0, nullptr);
+      const T2 d0 = interior<R, DIM, D>(g, c, u, (R)0, nullptr);
+      pdl_trigger();
+      Ds[p] = d0;
     } else {
-      exact::update<R>(c, stage, p, interior<R, DIM, FORM>(g, c, u, V[p], Ds + p), Psi, K, Yout);
+      const T2 f0 = interior<R, DIM, FORM>(g, c, u, V[p], Ds + p);
+      pdl_trigger();
+      exact::update<R>(c, stage, p, f0, Psi, K, Yout);
     }
     return;
   }
@@ -269,10 +279,7 @@ cudaError_t by_bc(const Geom& g, int BC, const Consts<R>& c, const ExactStageArg
   const Map m = make_map(g, NT);
   const unsigned blocks = m.shell_blocks + (m.deep + NT - 1) / NT;
   const dim3 gr(blocks), bl(NT);
-  // Launch overlap (PDL) hands out the next launch's blocks as the last ones
-  // end, which loads the SMs unevenly where a launch is a few blocks per SM
-  // (WIDE 32^3: 65 us a step with it, 50 without; 200^2 MSD 52 and 42).
-  const bool pdl = wide::g_pdl != 0 && (blocks <= 152 || blocks > 4096);
+  const bool pdl = wide::g_pdl != 0;
 #define NLSE_POINT(bc)                                                                          \
   case bc:                                                                                      \
     return launch_k(pass<R, DIM, FORM, bc, VAR, NT>, gr, bl, 0, st, pdl, g, c, a.Yin, a.Psi,  \

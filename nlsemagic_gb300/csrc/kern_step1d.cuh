@@ -26,6 +26,11 @@
 // per slot did not fit the instruction cache (2SHOC MSD on 1024 points, R = 8:
 // 13 us a step).
 //
+// The next launch (PDL) is triggered when a window is done, not at the start: its
+// blocks are then placed as this one's end, which hides its latency.  Placed at
+// the start they load the SMs unevenly (FP64 CD on 48611 points, one solve: 49 us a
+// step; 16.5 without overlap, 15.1 so).
+//
 // Slots outside the grid hold zeros; nothing inside reads them.  The state is
 // read from one buffer and written to another (neighbouring windows still
 // read the old one).
@@ -235,7 +240,6 @@ template <int METHOD, int BC, int R>
 __global__ void __launch_bounds__(32 * MAX_WARPS)
     mixed_steps(int n, Consts<float> c, const float2* hi_in, const float2* lo_in, const float* V,
                 float2* hi_out, float2* lo_out, Plan pl) {
-  pdl_trigger();  // the next kernel may launch; it waits for this one
   const int first = (int)(blockIdx.x * pl.warps + (threadIdx.x >> 5)) * pl.U;
   if (first >= n) return;
   pdl_wait();  // the previous kernel's output
@@ -250,7 +254,6 @@ __global__ void __launch_bounds__(32 * MAX_WARPS)
   using namespace exact;
   typedef C2<F> T2;
   constexpr int W = 32 * R;
-  pdl_trigger();  // the next kernel may launch; it waits for this one
   const int lane = (int)(threadIdx.x & 31);
   const int first = (int)(blockIdx.x * pl.warps + (threadIdx.x >> 5)) * pl.U;
   if (first >= n) return;
@@ -337,6 +340,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS)
       }
     }
   }
+  pdl_trigger();  // the next kernel may launch; it waits for this one
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int i = lane * R + r;
@@ -363,8 +367,8 @@ template <typename F, int VAR>
 cudaError_t launch_exact(const Geom& g, int method, int BC, const Consts<F>& c, const C2<F>* in,
                          const F* V, C2<F>* out, const Step1dShape& sh, int m, cudaStream_t st) {
 #define NLSE_STEP1D(R)                                                                     \
-  return method == 2 ? exact_by_bc<F, 2, R, VAR>(g, BC, c, in, V, out, m, sh.warps, st, sh.pdl) \
-                     : exact_by_bc<F, 1, R, VAR>(g, BC, c, in, V, out, m, sh.warps, st, sh.pdl)
+  return method == 2 ? exact_by_bc<F, 2, R, VAR>(g, BC, c, in, V, out, m, sh.warps, st, wide::g_pdl != 0) \
+                     : exact_by_bc<F, 1, R, VAR>(g, BC, c, in, V, out, m, sh.warps, st, wide::g_pdl != 0)
   switch (sh.per_lane) {
     case 1: NLSE_STEP1D(1);
     case 2: NLSE_STEP1D(2);

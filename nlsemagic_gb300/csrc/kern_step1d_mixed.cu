@@ -45,13 +45,8 @@ static cudaError_t mixed_by_bc(const Geom& g, int BC, const Consts<float>& c, co
 // 12.4 / 5.1, 16.5 / 11.1, -; R = 4, m = 1: -, -, -, 47 / 38.  2SHOC, 25.8 /
 // 8.8, 27 / 13.7, 45 / 18.3: R = 1, m = 1: 13.1 / 4.7, -, -; R = 2, m = 1:
 // -, 20 / 8.8, 28 / 17.4.
-//
-// Launch overlap (PDL) is left out for FP64 grids of more windows than SMs:
-// the next launch's blocks then take places as the last ones end, which fills
-// some SMs twice and leaves others idle for the whole launch (CD at 48611
-// points, R = 2, m = 1: 49 / 11.8 with it, 16.5 / 11.1 without).
 Step1dShape step1d_shape(const Geom& g, int method, int precision, int kernel_kind) {
-  Step1dShape sh = {0, 4, step1d::MAX_WARPS, wide::g_pdl != 0};
+  Step1dShape sh = {0, 4, step1d::MAX_WARPS};
   const long long n = g.n;
   if (g.ndim != 1 || kernel_kind != KERNEL_TILED || !wide::g_seg1d || n > (1LL << 30)) return sh;
   if (precision == 2) {
@@ -65,8 +60,6 @@ Step1dShape step1d_shape(const Geom& g, int method, int precision, int kernel_ki
     sh.steps = n <= (1LL << 13) ? 6 : (n <= (1LL << 16) ? 4 : 2);
   }
   if (n <= 32 * sh.per_lane) sh.steps = 1 << 16;  // one window, nothing lost
-  if (precision == 2 && step1d::make_plan(n, method, sh.per_lane, sh.steps, 1).blocks > 152)
-    sh.pdl = false;
   return sh;
 }
 
@@ -75,8 +68,8 @@ cudaError_t launch_step1d_mixed(const Geom& g, int method, int BC, const Consts<
                                 float2* l2, const Step1dShape& sh, int m, cudaStream_t st) {
 #define NLSE_STEP1D(R)                                                                            \
   return method == 2                                                                              \
-             ? step1d::mixed_by_bc<2, R>(g, BC, c, hi, lo, V, ho, l2, m, sh.warps, st, sh.pdl) \
-             : step1d::mixed_by_bc<1, R>(g, BC, c, hi, lo, V, ho, l2, m, sh.warps, st, sh.pdl)
+             ? step1d::mixed_by_bc<2, R>(g, BC, c, hi, lo, V, ho, l2, m, sh.warps, st, wide::g_pdl != 0) \
+             : step1d::mixed_by_bc<1, R>(g, BC, c, hi, lo, V, ho, l2, m, sh.warps, st, wide::g_pdl != 0)
   switch (sh.per_lane) {
     case 1: NLSE_STEP1D(1);
     case 2: NLSE_STEP1D(2);

@@ -171,6 +171,7 @@ __device__ __forceinline__ void mixed_tile(const Geom& g, const Consts<float>& c
 
 #pragma unroll
   for (int stage = 1; stage <= 4; ++stage) {
+    if (stage == 4) pdl_trigger();  // the next kernel may launch; it waits for this one
     const int m = (stage - 1) * H;  // margin of this stage's cells
     float2* const ein = stage & 1 ? ea : eb;
     float2* const eout = stage & 1 ? eb : ea;
@@ -291,7 +292,6 @@ __global__ void __launch_bounds__(XT* G, MINB)
   constexpr int H = Shape<METHOD, XT, G, R>::H;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* const sm = reinterpret_cast<float2*>(smem_raw);
-  pdl_trigger();  // the next kernel may launch; it waits for this one
   const Tile t = tile_of<H>(g, (int)blockIdx.x, (int)blockIdx.y, nbx, nby);
   pdl_wait();  // the previous kernel's output
   if (at_edge<H>(g, t))

@@ -61,6 +61,7 @@ __device__ __forceinline__ void exact_cd_tile(const Geom& g, const Consts<float>
 
 #pragma unroll
   for (int stage = 1; stage <= 4; ++stage) {
+    if (stage == 4) pdl_trigger();  // the next kernel may launch; it waits for this one
     const int m = stage - 1;  // margin of this stage's cells
     T2* const yin = stage & 1 ? ya : yb;
     T2* const yout = stage & 1 ? yb : ya;
@@ -133,7 +134,6 @@ __global__ void __launch_bounds__(XT* G, MINB)
                   int nbx, int nby) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C2<float>* const sm = reinterpret_cast<C2<float>*>(smem_raw);
-  pdl_trigger();  // the next kernel may launch; it waits for this one
   const Tile t = tile_of<1>(g, (int)blockIdx.x, (int)blockIdx.y, nbx, nby);
   pdl_wait();  // the previous kernel's output
   if (at_edge<1>(g, t))

@@ -49,9 +49,12 @@ static cudaError_t by_shape(const Geom& g, const Consts<float>& c, const float2*
 //   500^2    13.1 /  5.8      7.2 /  3.1                  8.1 /  3.8
 //   1300^2   38.8 / 47.5     20.0 / 17.3                 18.3 / 13.6
 // MSD adds two quotients one after the other to every stage of an edge tile,
-// which small grids wait for: CD stays with the stage launches up to 2^16
-// points (160^2: 7.7 / 3.3 against 7.8 / 3.3), 2SHOC takes 32 x 32 up to 2^18
-// (420^2: 15.2 / 7.0, SMALL 15.4 / 7.6, MIDDLE 13.4 / 6.4, LARGE 19 / 7.6).
+// which small grids wait for (CD 64^2: 7.2 / 2.6 -> 7.5 / 2.6, 250^2 10.3 / 3.8
+// -> 7.7 / 3.2); 2SHOC takes 32 x 32 up to 2^18 (420^2: 15.2 / 7.0, SMALL 15.4 /
+// 7.6, MIDDLE 13.4 / 6.4, LARGE 19 / 7.6).  The next launch (PDL) is triggered
+// before the last stage: triggered at the start, its blocks are placed while this
+// launch's come and go and load the SMs unevenly (300^2 CD three in flight 2.6,
+// 2.3 so).
 // A grid of fewer than 16 points a side fills too little of a tile (8000 x 8:
 // 3.8 against 5.4 with three in flight).
 int step2d_shape(const Geom& g, int method, int BC, int precision, int kernel_kind) {
@@ -60,10 +63,7 @@ int step2d_shape(const Geom& g, int method, int BC, int precision, int kernel_ki
   if (precision == 2 || (precision == 1 && method == 2) || BC > 3) return 0;
   if (g.M < 16 || g.N < 16 || g.N > 65535 * 20) return 0;  // tile rows: gridDim.y
   if (precision == 1) return g.n <= (1LL << 19) ? SMALL : LARGE;
-  if (method == 1) {
-    if (BC == 2 && g.n <= (1LL << 16)) return 0;
-    return g.n <= (1LL << 18) ? SMALL : (g.n <= (1LL << 20) ? MIDDLE : LARGE);
-  }
+  if (method == 1) return g.n <= (1LL << 18) ? SMALL : (g.n <= (1LL << 20) ? MIDDLE : LARGE);
   if (g.n <= (1LL << 15)) return MIDDLE;
   if (g.n <= (1LL << 17)) return SMALL;
   return BC == 2 && g.n <= (1LL << 18) ? MIDDLE : LARGE;

@@ -129,10 +129,9 @@ cudaError_t mass_hilo(const float2* hi, const float2* lo, long long n, double* o
                       cudaStream_t st);
 
 // The form a 1D solve's run takes: RK4 steps per launch (0: the stage
-// launches), points per lane, warps per block, launches overlapped (PDL).
+// launches), points per lane, warps per block.
 struct Step1dShape {
   int steps, per_lane, warps;
-  bool pdl;
 };
 Step1dShape step1d_shape(const Geom& g, int method, int precision, int kernel_kind);
 // Whole RK4 steps of a 1D solve in registers (kern_step1d.cuh): m <= sh.steps
