@@ -149,6 +149,11 @@ int NLSE3D_TAKE_STEPS_CUDA_MIXED(const double *Uoldr, const double *Uoldi, const
  * input, imaginary plane taken as zero, as the reference does). */
 int nlse_take_steps(const nlse_problem *p, const double *Ur, const double *Ui, const double *V,
                     double *out_r, double *out_i, int chunk_size);
+/* The same on interleaved complex arrays (re, im pairs, 2 n doubles; the layout
+ * of C99, Fortran and numpy): no split into planes on the host.  The result is
+ * what re + 1j * im gives in numpy's arithmetic. */
+int nlse_take_steps_complex(const nlse_problem *p, const double *U, const double *V, double *out,
+                            int chunk_size);
 
 /* ------------------------------------------------------------------------
  * Resident solver: state and potential stay in HBM between chunks.  No
@@ -221,6 +226,9 @@ long long nlse_batch_bytes_for(const nlse_problem *p);
  * NLSE_PREC_MIXED. */
 int nlse_batch_add(nlse_batch *b, const nlse_problem *p, const double *Ur, const double *Ui,
                    const double *V, long long nsteps, int *slot);
+/* The same with an interleaved complex array (see nlse_take_steps_complex). */
+int nlse_batch_add_complex(nlse_batch *b, const nlse_problem *p, const double *U, const double *V,
+                           long long nsteps, int *slot);
 /* Advance every unfinished solve by up to max_steps RK4 steps (one
  * persistent launch; asynchronous on the batch stream). */
 int nlse_batch_run(nlse_batch *b, int max_steps);
@@ -228,6 +236,7 @@ int nlse_batch_run(nlse_batch *b, int max_steps);
 int nlse_batch_remaining(nlse_batch *b, int slot, long long *steps_left);
 /* Copy a slot's state to host planar arrays (waits for queued work). */
 int nlse_batch_download(nlse_batch *b, int slot, double *Ur, double *Ui);
+int nlse_batch_download_complex(nlse_batch *b, int slot, double *U);
 /* Release a slot and its pool memory. */
 int nlse_batch_remove(nlse_batch *b, int slot);
 int nlse_batch_sync(nlse_batch *b);

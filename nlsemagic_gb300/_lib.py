@@ -80,6 +80,7 @@ SIGNATURES = {
     "nlse_version": (ctypes.c_char_p, []),
     "nlse_linear_stability_k": (_d, [_i, _i, _d, _d]),
     "nlse_take_steps": (_i, [ctypes.POINTER(Problem), _dp, _dp, _dp, _dp, _dp, _i]),
+    "nlse_take_steps_complex": (_i, [ctypes.POINTER(Problem), _dp, _dp, _dp, _i]),
     "nlse_solver_create": (_i, [ctypes.POINTER(Problem), ctypes.POINTER(_vp)]),
     "nlse_solver_destroy": (_i, [_vp]),
     "nlse_solver_upload": (_i, [_vp, _dp, _dp, _dp]),
@@ -108,6 +109,9 @@ SIGNATURES = {
     "nlse_batch_bytes_for": (_ll, [ctypes.POINTER(Problem)]),
     "nlse_batch_add": (_i, [_vp, ctypes.POINTER(Problem), _dp, _dp, _dp, _ll,
                             ctypes.POINTER(_i)]),
+    "nlse_batch_add_complex": (_i, [_vp, ctypes.POINTER(Problem), _dp, _dp, _ll,
+                                    ctypes.POINTER(_i)]),
+    "nlse_batch_download_complex": (_i, [_vp, _i, _dp]),
     "nlse_batch_run": (_i, [_vp, _i]),
     "nlse_batch_remaining": (_i, [_vp, _i, ctypes.POINTER(_ll)]),
     "nlse_batch_download": (_i, [_vp, _i, _dp, _dp]),

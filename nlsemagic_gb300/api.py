@@ -73,6 +73,11 @@ def planar(U):
     return re, im
 
 
+def _interleaved(U):
+    """Whether U's memory is the interleaved complex array of the C ABI."""
+    return U.dtype == np.complex128 and U.flags.f_contiguous and U.flags.aligned
+
+
 def take_steps(U, V, s, a, h2, BC, chunk_size, k, method=1, precision=PREC_DOUBLE,
                flags=FLAG_MSD_GUARD):
     """Advance U by chunk_size RK4 steps on the GPU; returns the new U."""
@@ -82,8 +87,13 @@ def take_steps(U, V, s, a, h2, BC, chunk_size, k, method=1, precision=PREC_DOUBL
         raise ValueError("V must have the shape of U (%s vs %s)" % (V.shape, U.shape))
     ndim, dims = grid_dims(U.shape)
     prob = make_problem(ndim, dims, method, precision, BC, s, a, h2, k, flags)
-    re, im = planar(U)
     vv = np.ascontiguousarray(V.ravel(order="F"))
+    if _interleaved(U):
+        out = np.empty(U.size, dtype=np.complex128)
+        check(load().nlse_take_steps_complex(ctypes.byref(prob), _ptr(U), _ptr(vv), _ptr(out),
+                                             int(chunk_size)))
+        return out.reshape(U.shape, order="F")
+    re, im = planar(U)
     out_r = np.empty_like(re)
     out_i = np.empty_like(im)
     check(load().nlse_take_steps(ctypes.byref(prob), _ptr(re), _ptr(im), _ptr(vv), _ptr(out_r),
@@ -332,9 +342,14 @@ class Batch:
         U = np.asarray(U)
         ndim, dims = grid_dims(U.shape)
         p = make_problem(ndim, dims, method, precision, BC, s, a, h2, k, flags)
-        re, im = planar(U)
         vv = np.ascontiguousarray(np.asarray(V, dtype=np.float64).ravel(order="F"))
         slot = ctypes.c_int()
+        if _interleaved(U):
+            check(self._lib.nlse_batch_add_complex(self._h, ctypes.byref(p), _ptr(U), _ptr(vv),
+                                                   int(nsteps), ctypes.byref(slot)))
+            self.shapes[slot.value] = U.shape
+            return slot.value
+        re, im = planar(U)
         check(self._lib.nlse_batch_add(self._h, ctypes.byref(p), _ptr(re), _ptr(im), _ptr(vv),
                                        int(nsteps), ctypes.byref(slot)))
         self.shapes[slot.value] = U.shape
@@ -359,11 +374,9 @@ class Batch:
 
     def download(self, slot):
         shape = self.shapes[slot]
-        n = int(np.prod(shape))
-        re = np.empty(n)
-        im = np.empty(n)
-        check(self._lib.nlse_batch_download(self._h, int(slot), _ptr(re), _ptr(im)))
-        return (re + 1j * im).reshape(shape, order="F")
+        out = np.empty(int(np.prod(shape)), dtype=np.complex128)
+        check(self._lib.nlse_batch_download_complex(self._h, int(slot), _ptr(out)))
+        return out.reshape(shape, order="F")
 
     def remove(self, slot):
         check(self._lib.nlse_batch_remove(self._h, int(slot)))

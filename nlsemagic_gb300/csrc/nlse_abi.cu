@@ -513,19 +513,21 @@ static int ensure_stage(nlse_solver* s) {
 
 // Convert the planar doubles (re, im, V) already on the device into the
 // solver's internal layout.
-static int ingest(nlse_solver* s, const double* re, const double* im, const double* V) {
+// stride 2: re and im are the parts of an interleaved complex array.
+static int ingest(nlse_solver* s, const double* re, const double* im, const double* V,
+                  int stride = 1) {
   const long long n = s->g.n;
   switch (s->prob.precision) {
     case NLSE_PREC_DOUBLE:
-      CUDA_TRY(planar_to_c2d(re, im, (C2<double>*)s->psi, n, s->stream));
+      CUDA_TRY(planar_to_c2d(re, im, (C2<double>*)s->psi, n, s->stream, stride));
       if (V) CUDA_TRY(cudaMemcpyAsync(s->V, V, sizeof(double) * n, cudaMemcpyDefault, s->stream));
       break;
     case NLSE_PREC_SINGLE:
-      CUDA_TRY(planar_to_c2f(re, im, (C2<float>*)s->psi, n, s->stream));
+      CUDA_TRY(planar_to_c2f(re, im, (C2<float>*)s->psi, n, s->stream, stride));
       if (V) CUDA_TRY(real_to_float(V, (float*)s->V, n, s->stream));
       break;
     default:
-      CUDA_TRY(planar_to_hilo(re, im, s->hi[s->cur], s->lo[s->cur], n, s->stream));
+      CUDA_TRY(planar_to_hilo(re, im, s->hi[s->cur], s->lo[s->cur], n, s->stream, stride));
       if (V) CUDA_TRY(real_to_float(V, s->Vf, n, s->stream));
       s->strips_fresh = false;  // refilled before the next stage launch
       break;
@@ -602,17 +604,17 @@ extern "C" int nlse_solver_upload(nlse_solver* s, const double* Ur, const double
   return NLSE_OK;
 }
 
-static int emit(nlse_solver* s, double* re, double* im) {
+static int emit(nlse_solver* s, double* re, double* im, int stride = 1) {
   const long long n = s->g.n;
   switch (s->prob.precision) {
     case NLSE_PREC_DOUBLE:
-      CUDA_TRY(c2d_to_planar((const C2<double>*)s->psi, re, im, n, s->stream));
+      CUDA_TRY(c2d_to_planar((const C2<double>*)s->psi, re, im, n, s->stream, stride));
       break;
     case NLSE_PREC_SINGLE:
-      CUDA_TRY(c2f_to_planar((const C2<float>*)s->psi, re, im, n, s->stream));
+      CUDA_TRY(c2f_to_planar((const C2<float>*)s->psi, re, im, n, s->stream, stride));
       break;
     default:
-      CUDA_TRY(hilo_to_planar(s->hi[s->cur], s->lo[s->cur], re, im, n, s->stream));
+      CUDA_TRY(hilo_to_planar(s->hi[s->cur], s->lo[s->cur], re, im, n, s->stream, stride));
       break;
   }
   return NLSE_OK;
@@ -979,12 +981,9 @@ static bool same_layout(const nlse_problem& a, const nlse_problem& b) {
   return true;
 }
 
-extern "C" int nlse_take_steps(const nlse_problem* p, const double* Ur, const double* Ui,
-                               const double* V, double* out_r, double* out_i, int chunk_size) {
-  int rc = validate(p);
-  if (rc) return rc;
-  if (!Ur || !V || !out_r || !out_i) return fail(NLSE_ERR_ARG, "NULL array argument");
-  if (chunk_size < 0) return fail(NLSE_ERR_ARG, "chunk_size must be >= 0");
+// The calling thread's cached solver, made or refreshed for *p.
+static int cached_solver(const nlse_problem* p, nlse_solver** out) {
+  int rc = NLSE_OK;
   int dev = 0;
   CUDA_TRY(cudaGetDevice(&dev));
   nlse_solver* s = t_cache.s;
@@ -1006,10 +1005,48 @@ extern "C" int nlse_take_steps(const nlse_problem* p, const double* Ur, const do
     s->kernel_kind = (p->flags & NLSE_FLAG_GATHER) ? KERNEL_GATHER : KERNEL_TILED;
   }
   s->cur = 0;
-  rc = nlse_solver_upload(s, Ur, Ui, V);
+  *out = s;
+  return NLSE_OK;
+}
+
+extern "C" int nlse_take_steps(const nlse_problem* p, const double* Ur, const double* Ui,
+                               const double* V, double* out_r, double* out_i, int chunk_size) {
+  int rc = validate(p);
+  if (rc) return rc;
+  if (!Ur || !V || !out_r || !out_i) return fail(NLSE_ERR_ARG, "NULL array argument");
+  if (chunk_size < 0) return fail(NLSE_ERR_ARG, "chunk_size must be >= 0");
+  nlse_solver* s = nullptr;
+  rc = cached_solver(p, &s);
+  if (!rc) rc = nlse_solver_upload(s, Ur, Ui, V);
   if (!rc) rc = nlse_solver_run(s, chunk_size);
   if (!rc) rc = nlse_solver_download(s, out_r, out_i);
   return rc;
+}
+
+extern "C" int nlse_take_steps_complex(const nlse_problem* p, const double* U, const double* V,
+                                       double* out, int chunk_size) {
+  int rc = validate(p);
+  if (rc) return rc;
+  if (!U || !V || !out) return fail(NLSE_ERR_ARG, "NULL array argument");
+  if (chunk_size < 0) return fail(NLSE_ERR_ARG, "chunk_size must be >= 0");
+  nlse_solver* s = nullptr;
+  rc = cached_solver(p, &s);
+  if (!rc) rc = ensure_stage(s);
+  if (rc) return rc;
+  CUDA_TRY(cudaSetDevice(s->device));
+  const size_t n = (size_t)s->g.n, b = sizeof(double) * n;
+  CUDA_TRY(cudaMemcpyAsync(s->stage, U, 2 * b, cudaMemcpyHostToDevice, s->stream));
+  CUDA_TRY(cudaMemcpyAsync(s->stage + 2 * n, V, b, cudaMemcpyHostToDevice, s->stream));
+  rc = ingest(s, s->stage, s->stage + 1, s->stage + 2 * n, 2);
+  if (!rc) rc = nlse_solver_run(s, chunk_size);
+  if (!rc) rc = emit(s, s->stage, s->stage + 1, 2);
+  if (rc) {
+    cudaStreamSynchronize(s->stream);  // U and V may be page-locked: still being read
+    return rc;
+  }
+  CUDA_TRY(cudaMemcpyAsync(out, s->stage, 2 * b, cudaMemcpyDeviceToHost, s->stream));
+  CUDA_TRY(cudaStreamSynchronize(s->stream));
+  return device_error_check();
 }
 
 static nlse_problem mkprob(int ndim, long long M, long long N, long long L, int method,

@@ -235,8 +235,9 @@ static int ensure_stage(nlse_batch* b, size_t doubles) {
   return NLSE_OK;
 }
 
-extern "C" int nlse_batch_add(nlse_batch* b, const nlse_problem* p, const double* Ur,
-                              const double* Ui, const double* V, long long nsteps, int* slot) {
+// stride 2: Ur is an interleaved complex array, Ui = Ur + 1.
+static int add_solve(nlse_batch* b, const nlse_problem* p, const double* Ur, const double* Ui,
+                     int stride, const double* V, long long nsteps, int* slot) {
   if (!b || !p || !Ur || !V || !slot) return nlse::set_error(NLSE_ERR_ARG, "NULL argument");
   if (nsteps < 0) return nlse::set_error(NLSE_ERR_ARG, "nsteps must be >= 0");
   if (p->precision != NLSE_PREC_DOUBLE && p->precision != NLSE_PREC_MIXED)
@@ -294,21 +295,31 @@ extern "C" int nlse_batch_add(nlse_batch* b, const nlse_problem* p, const double
     S.used = false;
     return rc;
   }
-  double *re = b->stage, *im = b->stage + n, *vv = b->stage + 2 * n;
-  BTRY(cudaMemcpyAsync(re, Ur, sizeof(double) * n, cudaMemcpyHostToDevice, b->stream));
-  if (Ui) BTRY(cudaMemcpyAsync(im, Ui, sizeof(double) * n, cudaMemcpyHostToDevice, b->stream));
+  double *re = b->stage, *im = b->stage + (stride == 2 ? 1 : n), *vv = b->stage + 2 * n;
+  BTRY(cudaMemcpyAsync(re, Ur, sizeof(double) * n * stride, cudaMemcpyHostToDevice, b->stream));
+  if (Ui && stride == 1)
+    BTRY(cudaMemcpyAsync(im, Ui, sizeof(double) * n, cudaMemcpyHostToDevice, b->stream));
   BTRY(cudaMemcpyAsync(vv, V, sizeof(double) * n, cudaMemcpyHostToDevice, b->stream));
   if (p->precision == NLSE_PREC_DOUBLE) {
-    BTRY(planar_to_c2d(re, Ui ? im : nullptr, (C2<double>*)S.d.buf[0], n, b->stream));
+    BTRY(planar_to_c2d(re, Ui ? im : nullptr, (C2<double>*)S.d.buf[0], n, b->stream, stride));
     BTRY(cudaMemcpyAsync(S.d.buf[4], vv, sizeof(double) * n, cudaMemcpyDeviceToDevice, b->stream));
   } else {
     BTRY(planar_to_hilo(re, Ui ? im : nullptr, (float2*)S.d.buf[0], (float2*)S.d.buf[2], n,
-                        b->stream));
+                        b->stream, stride));
     BTRY(real_to_float(vv, (float*)S.d.buf[7], n, b->stream));
   }
   BTRY(cudaStreamSynchronize(b->stream));  // host buffers reusable on return
   *slot = idx;
   return NLSE_OK;
+}
+
+extern "C" int nlse_batch_add(nlse_batch* b, const nlse_problem* p, const double* Ur,
+                              const double* Ui, const double* V, long long nsteps, int* slot) {
+  return add_solve(b, p, Ur, Ui, 1, V, nsteps, slot);
+}
+extern "C" int nlse_batch_add_complex(nlse_batch* b, const nlse_problem* p, const double* U,
+                                      const double* V, long long nsteps, int* slot) {
+  return add_solve(b, p, U, U ? U + 1 : nullptr, 2, V, nsteps, slot);
 }
 
 // One cooperative launch per precision class present; the classes run one
@@ -474,7 +485,8 @@ extern "C" int nlse_batch_remaining(nlse_batch* b, int slot, long long* steps_le
   return NLSE_OK;
 }
 
-extern "C" int nlse_batch_download(nlse_batch* b, int slot, double* Ur, double* Ui) {
+// stride 2: Ur takes the interleaved complex array.
+static int fetch(nlse_batch* b, int slot, double* Ur, double* Ui, int stride) {
   if (!b || !Ur || !Ui || slot < 0 || slot >= (int)b->slots.size() || !b->slots[slot].used)
     return nlse::set_error(NLSE_ERR_ARG, "bad slot or NULL array");
   int rc = nlse_batch_sync(b);
@@ -483,17 +495,26 @@ extern "C" int nlse_batch_download(nlse_batch* b, int slot, double* Ur, double* 
   const long long n = S.d.g.n;
   rc = ensure_stage(b, 2 * (size_t)n);
   if (rc) return rc;
+  double *re = b->stage, *im = b->stage + (stride == 2 ? 1 : n);
   if (S.d.prec == NLSE_PREC_DOUBLE) {
-    BTRY(c2d_to_planar((const C2<double>*)S.d.buf[0], b->stage, b->stage + n, n, b->stream));
+    BTRY(c2d_to_planar((const C2<double>*)S.d.buf[0], re, im, n, b->stream, stride));
   } else {
     int c = S.d.cur;
-    BTRY(hilo_to_planar((const float2*)S.d.buf[c], (const float2*)S.d.buf[2 + c], b->stage,
-                        b->stage + n, n, b->stream));
+    BTRY(hilo_to_planar((const float2*)S.d.buf[c], (const float2*)S.d.buf[2 + c], re, im, n,
+                        b->stream, stride));
   }
-  BTRY(cudaMemcpyAsync(Ur, b->stage, sizeof(double) * n, cudaMemcpyDeviceToHost, b->stream));
-  BTRY(cudaMemcpyAsync(Ui, b->stage + n, sizeof(double) * n, cudaMemcpyDeviceToHost, b->stream));
+  BTRY(cudaMemcpyAsync(Ur, re, sizeof(double) * n * stride, cudaMemcpyDeviceToHost, b->stream));
+  if (stride == 1)
+    BTRY(cudaMemcpyAsync(Ui, im, sizeof(double) * n, cudaMemcpyDeviceToHost, b->stream));
   BTRY(cudaStreamSynchronize(b->stream));
   return NLSE_OK;
+}
+
+extern "C" int nlse_batch_download(nlse_batch* b, int slot, double* Ur, double* Ui) {
+  return fetch(b, slot, Ur, Ui, 1);
+}
+extern "C" int nlse_batch_download_complex(nlse_batch* b, int slot, double* U) {
+  return fetch(b, slot, U, U ? U + 1 : nullptr, 2);
 }
 
 extern "C" int nlse_batch_remove(nlse_batch* b, int slot) {

@@ -105,19 +105,20 @@ long long mixed_fq_entries(const Geom& g, int method, int BC, int kernel_kind);
 long long exact_dsc_entries(const Geom& g, int method, int BC, int kernel_kind, bool single);
 long long mixed_dsc_entries(const Geom& g, int method, int BC, int kernel_kind);
 
-// Layout conversions and reductions (kern_util.cu).
+// Layout conversions and reductions (kern_util.cu).  stride 2: re and im are the
+// two parts of an interleaved complex array (im = re + 1).
 cudaError_t planar_to_c2d(const double* re, const double* im, C2<double>* out, long long n,
-                          cudaStream_t st);
+                          cudaStream_t st, int stride = 1);
 cudaError_t planar_to_c2f(const double* re, const double* im, C2<float>* out, long long n,
-                          cudaStream_t st);
+                          cudaStream_t st, int stride = 1);
 cudaError_t planar_to_hilo(const double* re, const double* im, float2* hi, float2* lo,
-                           long long n, cudaStream_t st);
+                           long long n, cudaStream_t st, int stride = 1);
 cudaError_t c2d_to_planar(const C2<double>* in, double* re, double* im, long long n,
-                          cudaStream_t st);
+                          cudaStream_t st, int stride = 1);
 cudaError_t c2f_to_planar(const C2<float>* in, double* re, double* im, long long n,
-                          cudaStream_t st);
+                          cudaStream_t st, int stride = 1);
 cudaError_t hilo_to_planar(const float2* hi, const float2* lo, double* re, double* im,
-                           long long n, cudaStream_t st);
+                           long long n, cudaStream_t st, int stride = 1);
 cudaError_t real_to_float(const double* in, float* out, long long n, cudaStream_t st);
 cudaError_t fill_zero_bytes(void* p, size_t bytes, cudaStream_t st);
 
