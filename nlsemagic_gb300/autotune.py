@@ -25,8 +25,8 @@ x faces' own lo, K and V from face-indexed arrays).
 Results are cached in a JSON file (``$NLSE_TUNE_CACHE`` or
 ``~/.cache/nlse_gb300/tune.json``) keyed by device name and problem class;
 :func:`apply` sets the knobs from the cache before a workload runs.  The
-knobs are process-wide and are read when a stage launch is issued or a graph
-captured, so they apply to solvers created afterwards.
+knobs are process-wide and are read when a run starts: a solver whose graphs
+were captured under other values captures them again.
 """
 from __future__ import annotations
 

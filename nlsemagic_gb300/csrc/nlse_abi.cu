@@ -7,6 +7,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "../../include/nlse_gb300.h"
@@ -49,8 +50,9 @@ int set_error(int code, const char* fmt, ...) {
 extern "C" const char* nlse_version(void) { return "nlse_gb300 1.0 (sm_103a)"; }
 
 // ---------------------------------------------------------------------------
-// tuning knobs (process-wide; read when a stage launch is issued or a graph is
-// captured, so they apply to solvers created or re-captured afterwards)
+// tuning knobs (process-wide; read when a launch is issued or a graph captured.
+// A run that finds a knob of the kernels' form changed since its graphs were
+// captured captures them again: a run never mixes forms)
 // ---------------------------------------------------------------------------
 namespace nlse {
 namespace wide {
@@ -68,6 +70,15 @@ namespace wide2d {
 extern int g_ty;
 }
 }  // namespace nlse
+// Changes of the knobs that choose between kernel forms.
+static std::atomic<unsigned> g_form_changes{0};
+static int set_form(int* knob, long long value) {
+  if (*knob != (int)value) {
+    *knob = (int)value;
+    ++g_form_changes;
+  }
+  return NLSE_OK;
+}
 static int g_default_graph_steps = 8;
 // Host arrays in page-locked (device-mapped) memory are read and written by
 // the layout-conversion kernels in place, over the host link, instead of
@@ -84,13 +95,11 @@ extern "C" int nlse_tune_set(const char* key, long long value) {
   if (!key) return fail(NLSE_ERR_ARG, "key is NULL");
   if (!strcmp(key, "wide.zc")) {
     if (value < 0 || value > (1 << 20)) return fail(NLSE_ERR_ARG, "wide.zc out of range");
-    nlse::wide::g_zc_override = (int)value;
-    return NLSE_OK;
+    return set_form(&nlse::wide::g_zc_override, value);
   }
   if (!strcmp(key, "wide2d")) {
     if (value != 0 && value != 1) return fail(NLSE_ERR_ARG, "wide2d must be 0 or 1");
-    nlse::wide::g_wide2d = (int)value;
-    return NLSE_OK;
+    return set_form(&nlse::wide::g_wide2d, value);
   }
   if (!strcmp(key, "io.zero_copy")) {
     if (value != 0 && value != 1) return fail(NLSE_ERR_ARG, "io.zero_copy must be 0 or 1");
@@ -99,45 +108,37 @@ extern "C" int nlse_tune_set(const char* key, long long value) {
   }
   if (!strcmp(key, "seg1d")) {
     if (value != 0 && value != 1) return fail(NLSE_ERR_ARG, "seg1d must be 0 or 1");
-    nlse::wide::g_seg1d = (int)value;
-    return NLSE_OK;
+    return set_form(&nlse::wide::g_seg1d, value);
   }
   if (!strcmp(key, "wide2d.ty")) {
     if (value != 0 && value != 8 && value != 16 && value != 32)
       return fail(NLSE_ERR_ARG, "wide2d.ty must be 0, 8, 16 or 32");
-    nlse::wide2d::g_ty = (int)value;
-    return NLSE_OK;
+    return set_form(&nlse::wide2d::g_ty, value);
   }
   if (!strcmp(key, "wide.z2")) {
     if (value != 0 && value != 1) return fail(NLSE_ERR_ARG, "wide.z2 must be 0 or 1");
-    nlse::wide::g_z2 = (int)value;
-    return NLSE_OK;
+    return set_form(&nlse::wide::g_z2, value);
   }
   if (!strcmp(key, "wide.ty")) {
     if (value != 4 && value != 8 && value != 16)
       return fail(NLSE_ERR_ARG, "wide.ty must be 4, 8 or 16");
-    nlse::wide::g_wide_ty = (int)value;
-    return NLSE_OK;
+    return set_form(&nlse::wide::g_wide_ty, value);
   }
   if (!strcmp(key, "wide.tile_order")) {
     if (value != 0 && value != 1) return fail(NLSE_ERR_ARG, "wide.tile_order must be 0 or 1");
-    nlse::wide::g_tile_order = (int)value;
-    return NLSE_OK;
+    return set_form(&nlse::wide::g_tile_order, value);
   }
   if (!strcmp(key, "face.blocks_per_sm")) {
     if (value < 1 || value > 64) return fail(NLSE_ERR_ARG, "face.blocks_per_sm out of range");
-    nlse::wide::g_face_bps = (int)value;
-    return NLSE_OK;
+    return set_form(&nlse::wide::g_face_bps, value);
   }
   if (!strcmp(key, "wide.pdl")) {
     if (value != 0 && value != 1) return fail(NLSE_ERR_ARG, "wide.pdl must be 0 or 1");
-    nlse::wide::g_pdl = (int)value;
-    return NLSE_OK;
+    return set_form(&nlse::wide::g_pdl, value);
   }
   if (!strcmp(key, "wide.strips")) {
     if (value != 0 && value != 1) return fail(NLSE_ERR_ARG, "wide.strips must be 0 or 1");
-    nlse::wide::g_strips = (int)value;
-    return NLSE_OK;
+    return set_form(&nlse::wide::g_strips, value);
   }
   if (!strcmp(key, "small1d.max_points")) {
     if (value < 0 || value > 65536) return fail(NLSE_ERR_ARG, "small1d.max_points out of range");
@@ -383,6 +384,7 @@ struct nlse_solver {
   int graph_steps;
   cudaGraphExec_t gexec[2];  // by the buffer the state is in before (cur, flip)
   int gflip[2];              // exact classes: the graph leaves it in the other one
+  unsigned form;             // g_form_changes when they were captured
   size_t bytes;
 };
 
@@ -825,6 +827,14 @@ extern "C" int nlse_solver_run(nlse_solver* s, long long nsteps) {
   const Step1dShape sh =
       step1d_shape(s->g, s->prob.method, s->prob.precision, s->kernel_kind);
   if (sh.steps) return run_step1d(s, sh, nsteps);
+  // Graphs of another form do not keep what the launches beside them rely on
+  // (3D mixed: the x-face strips of lo, which steps by point leave behind)
+  const unsigned form = g_form_changes;
+  if (s->form != form) {
+    if (s->gexec[0] || s->gexec[1]) CUDA_TRY(cudaStreamSynchronize(s->stream));
+    free_graphs(s);
+    s->form = form;
+  }
   if (s->g.ndim == 1 && s->g.n <= g_small1d_max && s->prob.precision != NLSE_PREC_DOUBLE &&
       (s->prob.method == 1 || s->dsc) && nsteps > 0)
     return run_small1d(s, nsteps);
