@@ -33,9 +33,12 @@ static bool point_path(const Geom& g, int method, int BC, int kernel_kind, bool 
 
 // D scratch: 2SHOC in gather form and by point.  FP32 2D grids on the tile
 // kernel take none; should the knob turn it off later, the gather kernel
-// recomputes D.
-long long exact_dsc_entries(const Geom& g, int method, int BC, int kernel_kind, bool single) {
+// recomputes D.  The contracted class takes the wide form by point, without D
+// (kern_exact_fma.cu).
+long long exact_dsc_entries(const Geom& g, int method, int BC, int kernel_kind, bool single,
+                            bool contracted) {
   if (method != 2) return 0;
+  if (contracted && point_path(g, method, BC, kernel_kind, false)) return 0;
   return tile2d_path(g, method, BC, kernel_kind, single) ? 0 : g.n;
 }
 

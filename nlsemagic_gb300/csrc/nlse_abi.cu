@@ -468,7 +468,8 @@ extern "C" int nlse_solver_create(const nlse_problem* p, nlse_solver** out) {
     if (!r) r = dalloc(s, &s->yb, 2 * es * n);
     if (!r) r = dalloc(s, &s->V, es * n);
     const long long nd = exact_dsc_entries(s->g, p->method, p->bc, s->kernel_kind,
-                                           p->precision == NLSE_PREC_SINGLE);
+                                           p->precision == NLSE_PREC_SINGLE,
+                                           (p->flags & NLSE_FLAG_FMA) != 0);
     if (!r && nd) r = dalloc(s, &s->dsc, 2 * es * nd);
   } else {
     for (int t = 0; t < 2 && !r; ++t) {
@@ -921,7 +922,8 @@ extern "C" long long nlse_solver_bytes_for(const nlse_problem* p) {
   if (p->precision == NLSE_PREC_DOUBLE || p->precision == NLSE_PREC_SINGLE) {
     const long long es = p->precision == NLSE_PREC_DOUBLE ? 8 : 4;
     b = 4 * 2 * es * n + es * n +
-        2 * es * exact_dsc_entries(g, p->method, p->bc, kind, p->precision == NLSE_PREC_SINGLE);
+        2 * es * exact_dsc_entries(g, p->method, p->bc, kind, p->precision == NLSE_PREC_SINGLE,
+                                   (p->flags & NLSE_FLAG_FMA) != 0);
   } else {
     const long long ng = mixed_ghost_entries(g, p->method, p->bc, kind);
     b = 8 * 8 * n + 4 * n + 16 * ng + 8 * mixed_fq_entries(g, p->method, p->bc, kind) +
@@ -981,10 +983,11 @@ static bool same_scalars(const nlse_problem& a, const nlse_problem& b) {
 }
 
 // Same device buffers: grid, precision, and what the stage kernels allocate
-// scratch for (method, boundary code, kernel kind).
+// scratch for (method, boundary code, kernel kind, contraction).
 static bool same_layout(const nlse_problem& a, const nlse_problem& b) {
+  const int kinds = NLSE_FLAG_GATHER | NLSE_FLAG_FMA;
   if (a.ndim != b.ndim || a.precision != b.precision || a.method != b.method || a.bc != b.bc ||
-      (a.flags & NLSE_FLAG_GATHER) != (b.flags & NLSE_FLAG_GATHER))
+      (a.flags & kinds) != (b.flags & kinds))
     return false;
   for (int d = 0; d < a.ndim; ++d)
     if (a.dims[d] != b.dims[d]) return false;

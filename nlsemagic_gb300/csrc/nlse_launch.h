@@ -101,8 +101,9 @@ int exact_stage_launches(const Geom& g, int method, int BC, int kernel_kind, boo
 long long mixed_ghost_entries(const Geom& g, int method, int BC, int kernel_kind);
 long long mixed_fq_entries(const Geom& g, int method, int BC, int kernel_kind);
 // Points of D scratch (ExactStageArgs / MixedStageArgs ::dsc) a 2SHOC stage
-// uses that takes two launches, else 0.
-long long exact_dsc_entries(const Geom& g, int method, int BC, int kernel_kind, bool single);
+// uses that takes two launches, else 0.  contracted: NLSE_FLAG_FMA.
+long long exact_dsc_entries(const Geom& g, int method, int BC, int kernel_kind, bool single,
+                            bool contracted);
 long long mixed_dsc_entries(const Geom& g, int method, int BC, int kernel_kind);
 
 // Layout conversions and reductions (kern_util.cu).  stride 2: re and im are the

@@ -211,7 +211,8 @@ class Server:
                 keep = []
                 for r in wait_solo:
                     i = r.inst
-                    need = Solver.bytes_for(i.U.shape, i.method, i.precision, i.BC)
+                    flags = solve_flags(i, self.fp64_fma)
+                    need = Solver.bytes_for(i.U.shape, i.method, i.precision, i.BC, flags)
                     if need > self.solo_bytes:
                         rejected.append(r.rid)
                         continue
@@ -219,7 +220,7 @@ class Server:
                         keep.append(r)  # waits for a large solve to retire
                         continue
                     sv = Solver(i.U.shape, method=i.method, precision=i.precision, BC=i.BC, s=i.s,
-                                a=i.a, h2=i.h * i.h, k=i.k, flags=solve_flags(i, self.fp64_fma))
+                                a=i.a, h2=i.h * i.h, k=i.k, flags=flags)
                     sv.upload(i.U, i.V)
                     solos.append(_Solo(r, clock(), sv, int(i.steps), need))
                     solo_used += need

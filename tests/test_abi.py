@@ -108,6 +108,21 @@ def test_bytes_for_counts_the_x_face_strips(lib):
     assert ghosts > 0 and ghosts % 16 == 0, (mixed, cd)
 
 
+def test_contracted_class_needs_no_d_scratch(lib):
+    # NLSE_FLAG_FMA: 2SHOC by point in 2D and 3D never forms D (16 bytes a
+    # point); in 1D, and in gather form, it does
+    fma = ng.FLAG_MSD_GUARD | ng.FLAG_FMA
+    for shape in ((40, 30, 20), (40, 31)):
+        n = int(np.prod(shape))
+        for BC in (1, 2, 3):
+            args = dict(method=2, precision=ng.PREC_DOUBLE, BC=BC)
+            lean = ng.Solver.bytes_for(shape, flags=fma, **args)
+            assert lean == ng.Solver.bytes_for(shape, **dict(args, method=1)), (shape, BC)
+            assert ng.Solver.bytes_for(shape, flags=fma | ng.FLAG_GATHER, **args) == lean + 16 * n
+    a = ng.Solver.bytes_for((500,), method=2, precision=ng.PREC_DOUBLE, BC=4, flags=fma)
+    assert a == ng.Solver.bytes_for((500,), method=2, precision=ng.PREC_DOUBLE, BC=4)
+
+
 def test_autotune_candidates_per_class():
     from nlsemagic_gb300 import autotune
     two = autotune.candidates((256, 256), 3)
