@@ -91,6 +91,12 @@ typedef struct nlse_problem {
  * their own on a contracted copy of the batch kernel);
  * nlse_take_steps_noalloc computes without contraction. */
 #define NLSE_FLAG_FMA 4
+/* 3D: the streaming kernels (z planes through shared memory) at every size, for
+ * the classes that have them (FP32, mixed; FP64 with 2SHOC, uncontracted), in
+ * place of stages by point.  Same bits.  2SHOC in FP64 and FP32 then needs no
+ * D scratch: 16 and 8 bytes a point less (72 and 36 held), slower by up to 2x.
+ * A solve without the flag whose scratch does not fit takes that form too. */
+#define NLSE_FLAG_STREAM 8
 
 const char *nlse_last_error_string(void);
 const char *nlse_version(void);
@@ -197,7 +203,9 @@ int nlse_solver_launches_per_step(const nlse_solver *s);
 /* Bytes of device memory held by the solver. */
 long long nlse_solver_device_bytes(const nlse_solver *s);
 /* Bytes of device memory a solver for *p holds after a host upload (its
- * state, scratch and planar staging buffers); -1 for an invalid problem.
+ * state, scratch and planar staging buffers); -1 for an invalid problem.  Where
+ * they do not fit, FP64 and FP32 3D 2SHOC solves hold what they do with
+ * NLSE_FLAG_STREAM.
  * For admission by a device-memory budget (no reference counterpart). */
 long long nlse_solver_bytes_for(const nlse_problem *p);
 

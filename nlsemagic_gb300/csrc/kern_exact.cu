@@ -7,7 +7,7 @@ namespace nlse {
 
 static bool tile2d_path(const Geom& g, int method, int BC, int kernel_kind, bool single) {
   (void)method;
-  return g.ndim == 2 && single && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_wide2d;
+  return g.ndim == 2 && single && kernel_kind != KERNEL_GATHER && BC != 4 && wide::g_wide2d;
 }
 
 // Thread-per-point stages (kern_point.cuh).  FP64 takes them in 2D and 3D: its
@@ -26,9 +26,10 @@ static bool tile2d_path(const Geom& g, int method, int BC, int kernel_kind, bool
 // 248 -> 127 / 123), and with MSD (160^3 186 / 145 -> 147 / 140; Dirichlet 168 /
 // 131 against 146 / 140 stays tiled).
 static bool point_path(const Geom& g, int method, int BC, int kernel_kind, bool single) {
-  if (kernel_kind != KERNEL_TILED || BC > 3) return false;
-  if (!single) return g.ndim >= 2;
-  return g.ndim == 3 && (method == 2 || BC == 2 || g.M % 2 || g.n <= (1LL << 20));
+  if (kernel_kind == KERNEL_GATHER || BC > 3) return false;
+  if (!single && (g.ndim == 2 || method == 1)) return g.ndim >= 2;
+  if (g.ndim != 3 || kernel_kind == KERNEL_STREAM) return false;
+  return !single || (method == 2 || BC == 2 || g.M % 2 || g.n <= (1LL << 20));
 }
 
 // D scratch: 2SHOC in gather form and by point.  FP32 2D grids on the tile
@@ -38,15 +39,21 @@ static bool point_path(const Geom& g, int method, int BC, int kernel_kind, bool 
 long long exact_dsc_entries(const Geom& g, int method, int BC, int kernel_kind, bool single,
                             bool contracted) {
   if (method != 2) return 0;
-  if (contracted && point_path(g, method, BC, kernel_kind, false)) return 0;
+  if (contracted && g.ndim >= 2 && kernel_kind != KERNEL_GATHER) return 0;
+  if (g.ndim == 3 && kernel_kind == KERNEL_STREAM) return 0;
   return tile2d_path(g, method, BC, kernel_kind, single) ? 0 : g.n;
+}
+
+// 3D: the tiled kernels (kern_tiled.cuh) form D on the way.
+bool exact_dsc_spare(const Geom& g, int method, int BC, int kernel_kind) {
+  return method == 2 && g.ndim == 3 && BC <= 3 && kernel_kind != KERNEL_GATHER;
 }
 
 int exact_stage_launches(const Geom& g, int method, int BC, int kernel_kind, bool single,
                          bool has_dsc) {
   if (tile2d_path(g, method, BC, kernel_kind, single)) return 1;
   if (seg1d_exact_path(g, method, BC, kernel_kind, single)) return 1;
-  if (kernel_kind == KERNEL_TILED && tiled_supported(g, g.ndim) && BC != 4 &&
+  if (kernel_kind != KERNEL_GATHER && tiled_supported(g, g.ndim) && BC != 4 &&
       !point_path(g, method, BC, kernel_kind, single))
     return 1;
   return method == 2 && has_dsc ? 2 : 1;  // (D,) F
@@ -56,7 +63,7 @@ template <typename R>
 cudaError_t launch_exact_stage(const Geom& g, int method, int BC, const Consts<R>& c,
                                const ExactStageArgs<R>& a, int stage, cudaStream_t st,
                                int kernel_kind) {
-  // (the allocation-free call has no D scratch: its 2SHOC forms D on the way)
+  // (2SHOC whose D scratch did not fit forms D on the way)
   if (point_path(g, method, BC, kernel_kind, sizeof(R) == 4) && (method == 1 || a.dsc))
     return launch_point_exact<R>(g, method, BC, c, a, stage, st);
   return launch_exact_stage_var<R, 0>(g, method, BC, c, a, stage, st, kernel_kind);

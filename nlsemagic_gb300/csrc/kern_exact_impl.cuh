@@ -18,17 +18,17 @@
 namespace nlse {
 
 inline bool seg1d_exact_path(const Geom& g, int method, int BC, int kernel_kind, bool single) {
-  return g.ndim == 1 && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_seg1d &&
+  return g.ndim == 1 && kernel_kind != KERNEL_GATHER && BC != 4 && wide::g_seg1d &&
          ((method == 2 && single) || g.n < (1LL << 22));
 }
 
 template <typename R, int DIM, int METHOD, int BC, int VAR>
 cudaError_t launch_one(const Geom& g, const Consts<R>& c, const ExactStageArgs<R>& a,
                               int stage, cudaStream_t st, int kernel_kind) {
-  // 3D, what does not go by point (kern_exact.cu): FP32 with CD, and FP64
-  // 2SHOC without D scratch
-  if constexpr (VAR == 0 && DIM == 3 && BC != 4 && (sizeof(R) == 4) == (METHOD == 1)) {
-    if (kernel_kind == KERNEL_TILED && tiled_supported(g, DIM))
+  // 3D, what does not go by point (kern_exact.cu): FP32 with CD, and 2SHOC
+  // without D scratch
+  if constexpr (VAR == 0 && DIM == 3 && BC != 4 && (sizeof(R) == 4 || METHOD == 2)) {
+    if (kernel_kind != KERNEL_GATHER && tiled_supported(g, DIM))
       return tiled::launch_exact<R, DIM, METHOD, BC>(g, c, a, stage, st);
   }
   // FP64 1D grids above the step kernel's limit (kern_step1d.cuh): staged
@@ -43,7 +43,7 @@ cudaError_t launch_one(const Geom& g, const Consts<R>& c, const ExactStageArgs<R
   // launch).  FP64 stays on the gather kernels, bound by FP64 issue, where
   // the tile's D on the halo costs more than the D scratch.
   if constexpr (DIM == 2 && std::is_same<R, float>::value) {
-    if (kernel_kind == KERNEL_TILED && BC != 4 && wide::g_wide2d)
+    if (kernel_kind != KERNEL_GATHER && BC != 4 && wide::g_wide2d)
       return tile2d::launch<R, METHOD, BC == 4 ? 1 : BC>(g, c, a, stage, st, wide::g_pdl != 0);
   }
   long long blocks = (g.n + 255) / 256;

@@ -36,9 +36,9 @@ int g_ty = 0;
 template <int DIM, int METHOD, int BC>
 static cudaError_t launch_one(const Geom& g, const Consts<float>& c, const MixedStageArgs& a,
                               int stage, cudaStream_t st, int kernel_kind) {
-  if (DIM == 2 && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_wide2d)
+  if (DIM == 2 && kernel_kind != KERNEL_GATHER && BC != 4 && wide::g_wide2d)
     return wide2d::launch<METHOD, BC == 4 ? 1 : BC>(g, a, c, stage, st, wide::g_pdl != 0);
-  if (kernel_kind == KERNEL_TILED && tiled_supported(g, DIM) && DIM == 3 && BC != 4) {
+  if (kernel_kind != KERNEL_GATHER && tiled_supported(g, DIM) && DIM == 3 && BC != 4) {
     tiled::MixedPol::Args A{a, c, stage, tiled::error_word()};
     return wide::launch<METHOD, BC == 4 ? 1 : BC>(g, A, st);
   }
@@ -74,7 +74,7 @@ static cudaError_t by_bc(const Geom& g, int BC, const Consts<float>& c, const Mi
 }
 
 static bool wide_path(const Geom& g, int BC, int kernel_kind) {
-  return kernel_kind == KERNEL_TILED && g.ndim == 3 && tiled_supported(g, 3) && BC != 4;
+  return kernel_kind != KERNEL_GATHER && g.ndim == 3 && tiled_supported(g, 3) && BC != 4;
 }
 
 // 3D stages by point (kern_point_mixed.cu): small grids, and grids whose rows
@@ -88,7 +88,8 @@ static bool wide_path(const Geom& g, int BC, int kernel_kind) {
 // streaming kernels choose those kernels; grids 3 cells thin, all face, stay
 // with them too.
 bool mixed_point_path(const Geom& g, int method, int BC, int kernel_kind) {
-  if (!wide_path(g, BC, kernel_kind) || g.M < 4 || g.N < 4 || g.L < 4) return false;
+  if (!wide_path(g, BC, kernel_kind) || kernel_kind == KERNEL_STREAM) return false;
+  if (g.M < 4 || g.N < 4 || g.L < 4) return false;
   if (!wide::g_pdl || !wide::g_strips || !wide::g_z2 || !wide::g_tile_order) return false;
   return g.M % 2 || g.n <= (method == 1 ? 3LL << 18 : 1LL << 20);
 }
@@ -123,8 +124,8 @@ cudaError_t mixed_strip_fill(const Geom& g, const float2* lo, const float* V, fl
 }
 
 int mixed_stage_launches(const Geom& g, int method, int BC, int kernel_kind, bool has_dsc) {
-  if (g.ndim == 2 && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_wide2d) return 1;
-  if (g.ndim == 1 && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_seg1d) return 1;
+  if (g.ndim == 2 && kernel_kind != KERNEL_GATHER && BC != 4 && wide::g_wide2d) return 1;
+  if (g.ndim == 1 && kernel_kind != KERNEL_GATHER && BC != 4 && wide::g_seg1d) return 1;
   if (mixed_point_path(g, method, BC, kernel_kind)) return 1;
   if (!wide_path(g, BC, kernel_kind)) return method == 2 && has_dsc ? 2 : 1;  // (D,) F
   return method == 2 ? 3 : 2;  // (ghosts,) interior, faces
@@ -135,7 +136,7 @@ int mixed_stage_launches(const Geom& g, int method, int BC, int kernel_kind, boo
 // that kernel off later, the gather kernel recomputes D instead.
 long long mixed_dsc_entries(const Geom& g, int method, int BC, int kernel_kind) {
   if (method != 2 || wide_path(g, BC, kernel_kind)) return 0;
-  if (g.ndim == 2 && kernel_kind == KERNEL_TILED && BC != 4 && wide::g_wide2d) return 0;
+  if (g.ndim == 2 && kernel_kind != KERNEL_GATHER && BC != 4 && wide::g_wide2d) return 0;
   return g.n;
 }
 

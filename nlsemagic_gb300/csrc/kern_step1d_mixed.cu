@@ -48,7 +48,7 @@ static cudaError_t mixed_by_bc(const Geom& g, int BC, const Consts<float>& c, co
 Step1dShape step1d_shape(const Geom& g, int method, int precision, int kernel_kind) {
   Step1dShape sh = {0, 4, step1d::MAX_WARPS};
   const long long n = g.n;
-  if (g.ndim != 1 || kernel_kind != KERNEL_TILED || !wide::g_seg1d || n > (1LL << 30)) return sh;
+  if (g.ndim != 1 || kernel_kind == KERNEL_GATHER || !wide::g_seg1d || n > (1LL << 30)) return sh;
   if (precision == 2) {
     if (n > (1LL << 16)) return sh;
     sh.warps = 1;

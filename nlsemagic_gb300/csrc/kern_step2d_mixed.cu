@@ -59,7 +59,7 @@ static cudaError_t by_shape(const Geom& g, const Consts<float>& c, const float2*
 // 3.8 against 5.4 with three in flight).
 int step2d_shape(const Geom& g, int method, int BC, int precision, int kernel_kind) {
   using namespace step2d;
-  if (g.ndim != 2 || kernel_kind != KERNEL_TILED || !wide::g_wide2d || wide2d::g_ty) return 0;
+  if (g.ndim != 2 || kernel_kind == KERNEL_GATHER || !wide::g_wide2d || wide2d::g_ty) return 0;
   if (precision == 2 || (precision == 1 && method == 2) || BC > 3) return 0;
   if (g.M < 16 || g.N < 16 || g.N > 65535 * 20) return 0;  // tile rows: gridDim.y
   if (precision == 1) return g.n <= (1LL << 19) ? SMALL : LARGE;

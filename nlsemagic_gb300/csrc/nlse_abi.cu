@@ -261,6 +261,11 @@ static Geom make_geom(const nlse_problem* p) {
   return g;
 }
 
+static int kind_of(const nlse_problem* p) {
+  if (p->flags & NLSE_FLAG_GATHER) return KERNEL_GATHER;
+  return (p->flags & NLSE_FLAG_STREAM) ? KERNEL_STREAM : KERNEL_TILED;
+}
+
 // Scalars in the precision and with the expressions of each reference file.
 static Consts<double> consts_double(const nlse_problem* p) {
   Consts<double> c;
@@ -362,7 +367,8 @@ struct nlse_solver {
   int kernel_kind;
   // exact precisions
   void *psi, *K, *ya, *yb, *V;
-  void* dsc;  // 2SHOC on the gather path: D scratch (C2<R> or float2 per point)
+  void* dsc;  // 2SHOC by gather or by point: D scratch (C2<R> or float2 per point)
+  size_t dsc_spare;  // its bytes where the solve also runs without it, else 0
   int flip;   // psi and ya are swapped (step launches write the state to the other buffer)
   // mixed precision
   float2 *hi[2], *lo[2], *mK, *da, *db, *dc, *fq;
@@ -395,8 +401,30 @@ static int device_error_check() {
   return NLSE_OK;
 }
 
+static void free_graphs(nlse_solver* s) {
+  for (int t = 0; t < 2; ++t) {
+    if (s->gexec[t]) cudaGraphExecDestroy(s->gexec[t]);
+    s->gexec[t] = nullptr;
+  }
+}
+
+// Gives the D scratch back where the solve has a form without it: what does not
+// fit beside it comes first.
+static bool drop_spare(nlse_solver* s) {
+  if (!s->dsc_spare) return false;
+  cudaGetLastError();  // of the allocation that failed
+  cudaStreamSynchronize(s->stream);
+  free_graphs(s);
+  cudaFree(s->dsc);
+  s->dsc = nullptr;
+  s->bytes -= s->dsc_spare;
+  s->dsc_spare = 0;
+  return true;
+}
+
 static int dalloc(nlse_solver* s, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && drop_spare(s)) e = cudaMalloc(p, bytes);
   if (e != cudaSuccess) {
     *p = nullptr;
     cudaGetLastError();
@@ -404,13 +432,6 @@ static int dalloc(nlse_solver* s, void** p, size_t bytes) {
   }
   s->bytes += bytes;
   return NLSE_OK;
-}
-
-static void free_graphs(nlse_solver* s) {
-  for (int t = 0; t < 2; ++t) {
-    if (s->gexec[t]) cudaGraphExecDestroy(s->gexec[t]);
-    s->gexec[t] = nullptr;
-  }
 }
 
 extern "C" int nlse_solver_destroy(nlse_solver* s) {
@@ -442,7 +463,7 @@ extern "C" int nlse_solver_create(const nlse_problem* p, nlse_solver** out) {
   s->g = make_geom(p);
   s->cd = consts_double(p);
   s->cf = p->precision == NLSE_PREC_MIXED ? consts_mixed(p) : consts_single(p);
-  s->kernel_kind = (p->flags & NLSE_FLAG_GATHER) ? KERNEL_GATHER : KERNEL_TILED;
+  s->kernel_kind = kind_of(p);
   s->graph_steps = g_default_graph_steps;
   cudaError_t e = cudaGetDevice(&s->device);
   if (e != cudaSuccess) {
@@ -470,7 +491,13 @@ extern "C" int nlse_solver_create(const nlse_problem* p, nlse_solver** out) {
     const long long nd = exact_dsc_entries(s->g, p->method, p->bc, s->kernel_kind,
                                            p->precision == NLSE_PREC_SINGLE,
                                            (p->flags & NLSE_FLAG_FMA) != 0);
-    if (!r && nd) r = dalloc(s, &s->dsc, 2 * es * nd);
+    if (!r && nd) {
+      r = dalloc(s, &s->dsc, 2 * es * nd);
+      if (exact_dsc_spare(s->g, p->method, p->bc, s->kernel_kind)) {
+        if (!r) s->dsc_spare = 2 * es * nd;
+        r = NLSE_OK;  // where it does not fit, the form without it
+      }
+    }
   } else {
     for (int t = 0; t < 2 && !r; ++t) {
       r = dalloc(s, (void**)&s->hi[t], sizeof(float2) * n);
@@ -917,7 +944,7 @@ extern "C" long long nlse_solver_bytes_for(const nlse_problem* p) {
   if (validate(p)) return -1;
   const Geom g = make_geom(p);
   const long long n = g.n;
-  const int kind = (p->flags & NLSE_FLAG_GATHER) ? KERNEL_GATHER : KERNEL_TILED;
+  const int kind = kind_of(p);
   long long b = 0;
   if (p->precision == NLSE_PREC_DOUBLE || p->precision == NLSE_PREC_SINGLE) {
     const long long es = p->precision == NLSE_PREC_DOUBLE ? 8 : 4;
@@ -985,7 +1012,7 @@ static bool same_scalars(const nlse_problem& a, const nlse_problem& b) {
 // Same device buffers: grid, precision, and what the stage kernels allocate
 // scratch for (method, boundary code, kernel kind, contraction).
 static bool same_layout(const nlse_problem& a, const nlse_problem& b) {
-  const int kinds = NLSE_FLAG_GATHER | NLSE_FLAG_FMA;
+  const int kinds = NLSE_FLAG_GATHER | NLSE_FLAG_FMA | NLSE_FLAG_STREAM;
   if (a.ndim != b.ndim || a.precision != b.precision || a.method != b.method || a.bc != b.bc ||
       (a.flags & kinds) != (b.flags & kinds))
     return false;
@@ -1015,7 +1042,7 @@ static int cached_solver(const nlse_problem* p, nlse_solver** out) {
     s->prob = *p;
     s->cd = consts_double(p);
     s->cf = p->precision == NLSE_PREC_MIXED ? consts_mixed(p) : consts_single(p);
-    s->kernel_kind = (p->flags & NLSE_FLAG_GATHER) ? KERNEL_GATHER : KERNEL_TILED;
+    s->kernel_kind = kind_of(p);
   }
   s->cur = 0;
   *out = s;

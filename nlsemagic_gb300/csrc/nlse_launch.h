@@ -10,7 +10,9 @@ struct nlse_ic;  // include/nlse_gb300.h
 
 namespace nlse {
 
-enum KernelKind { KERNEL_GATHER = 0, KERNEL_TILED = 1 };
+// STREAM: as TILED, but 3D stages by the streaming kernels where the class has
+// them, never by point (NLSE_FLAG_STREAM).
+enum KernelKind { KERNEL_GATHER = 0, KERNEL_TILED = 1, KERNEL_STREAM = 2 };
 
 template <typename R>
 struct ExactStageArgs {
@@ -104,6 +106,9 @@ long long mixed_fq_entries(const Geom& g, int method, int BC, int kernel_kind);
 // uses that takes two launches, else 0.  contracted: NLSE_FLAG_FMA.
 long long exact_dsc_entries(const Geom& g, int method, int BC, int kernel_kind, bool single,
                             bool contracted);
+// Whether a solve that uses that scratch has another form than the gather
+// kernels' without it (should it not fit).
+bool exact_dsc_spare(const Geom& g, int method, int BC, int kernel_kind);
 long long mixed_dsc_entries(const Geom& g, int method, int BC, int kernel_kind);
 
 // Layout conversions and reductions (kern_util.cu).  stride 2: re and im are the

@@ -49,7 +49,7 @@ from dataclasses import dataclass, field
 import numpy as np
 
 from .api import Batch, Solver
-from ._lib import (FLAG_FMA, FLAG_MSD_GUARD, NLSE_ERR_CAPACITY, PREC_DOUBLE,
+from ._lib import (FLAG_FMA, FLAG_MSD_GUARD, FLAG_STREAM, NLSE_ERR_CAPACITY, PREC_DOUBLE,
                    NLSEError)
 
 
@@ -213,6 +213,9 @@ class Server:
                     i = r.inst
                     flags = solve_flags(i, self.fp64_fma)
                     need = Solver.bytes_for(i.U.shape, i.method, i.precision, i.BC, flags)
+                    if need > self.solo_bytes:  # the form without D scratch
+                        flags |= FLAG_STREAM
+                        need = Solver.bytes_for(i.U.shape, i.method, i.precision, i.BC, flags)
                     if need > self.solo_bytes:
                         rejected.append(r.rid)
                         continue

@@ -123,6 +123,19 @@ def test_contracted_class_needs_no_d_scratch(lib):
     assert a == ng.Solver.bytes_for((500,), method=2, precision=ng.PREC_DOUBLE, BC=4)
 
 
+def test_stream_form_needs_no_d_scratch(lib):
+    # NLSE_FLAG_STREAM: FP64 and FP32 3D 2SHOC in the form that forms D on the way
+    shape, n = (40, 30, 20), 40 * 30 * 20
+    flags = ng.FLAG_MSD_GUARD | ng.FLAG_STREAM
+    for prec, es in ((ng.PREC_DOUBLE, 16), (ng.PREC_SINGLE, 8)):
+        args = dict(precision=prec, BC=2)
+        cd = ng.Solver.bytes_for(shape, method=1, **args)
+        assert ng.Solver.bytes_for(shape, method=2, flags=flags, **args) == cd
+        assert ng.Solver.bytes_for(shape, method=2, **args) == cd + es * n
+        two = ng.Solver.bytes_for((300, 20), method=2, **args)
+        assert ng.Solver.bytes_for((300, 20), method=2, flags=flags, **args) == two
+
+
 def test_autotune_candidates_per_class():
     from nlsemagic_gb300 import autotune
     two = autotune.candidates((256, 256), 3)
