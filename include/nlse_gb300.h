@@ -196,9 +196,9 @@ int nlse_solver_query(nlse_solver *s, int *idle);
 int nlse_solver_stream(nlse_solver *s, void **stream);
 /* Steps per captured CUDA graph (default 8; 0 disables graphs). */
 int nlse_solver_set_graph_steps(nlse_solver *s, int steps);
-/* Number of kernel launches one RK4 step takes stage by stage.  1D and 2D
- * solves run one or several whole steps per launch where that is faster (knobs
- * "seg1d", "wide2d.ty") and then enqueue fewer. */
+/* Number of kernel launches one RK4 step takes stage by stage; what 3D solves
+ * enqueue.  An upper bound in 1D and 2D, where a launch may run one or several
+ * whole steps (knobs "seg1d", "wide2d.ty"). */
 int nlse_solver_launches_per_step(const nlse_solver *s);
 /* Bytes of device memory held by the solver. */
 long long nlse_solver_device_bytes(const nlse_solver *s);

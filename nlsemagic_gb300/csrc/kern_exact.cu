@@ -52,7 +52,7 @@ bool exact_dsc_spare(const Geom& g, int method, int BC, int kernel_kind) {
 int exact_stage_launches(const Geom& g, int method, int BC, int kernel_kind, bool single,
                          bool has_dsc) {
   if (tile2d_path(g, method, BC, kernel_kind, single)) return 1;
-  if (seg1d_exact_path(g, method, BC, kernel_kind, single)) return 1;
+  if (!single && seg1d_exact_path(g, BC, kernel_kind)) return 1;
   if (kernel_kind != KERNEL_GATHER && tiled_supported(g, g.ndim) && BC != 4 &&
       !point_path(g, method, BC, kernel_kind, single))
     return 1;

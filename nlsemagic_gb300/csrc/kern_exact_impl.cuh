@@ -17,9 +17,10 @@
 
 namespace nlse {
 
-inline bool seg1d_exact_path(const Geom& g, int method, int BC, int kernel_kind, bool single) {
+// FP64 stage launches in staged segments
+inline bool seg1d_exact_path(const Geom& g, int BC, int kernel_kind) {
   return g.ndim == 1 && kernel_kind != KERNEL_GATHER && BC != 4 && wide::g_seg1d &&
-         ((method == 2 && single) || g.n < (1LL << 22));
+         g.n < (1LL << 22);
 }
 
 template <typename R, int DIM, int METHOD, int BC, int VAR>
@@ -35,7 +36,7 @@ cudaError_t launch_one(const Geom& g, const Consts<R>& c, const ExactStageArgs<R
   // segments, one launch per stage, below 2^22 points (bound by FP64 issue,
   // larger grids gain nothing)
   if constexpr (DIM == 1 && BC != 4 && sizeof(R) == 8) {
-    if (seg1d_exact_path(g, METHOD, BC, kernel_kind, false))
+    if (seg1d_exact_path(g, BC, kernel_kind))
       return seg1d::launch_exact<R, METHOD, BC, VAR>(g, c, a, stage, st, wide::g_pdl != 0);
   }
   // FP32 on 2D grids: the single-pass tile kernel (2SHOC 1.4-1.5x the

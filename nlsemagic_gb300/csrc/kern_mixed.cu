@@ -125,7 +125,6 @@ cudaError_t mixed_strip_fill(const Geom& g, const float2* lo, const float* V, fl
 
 int mixed_stage_launches(const Geom& g, int method, int BC, int kernel_kind, bool has_dsc) {
   if (g.ndim == 2 && kernel_kind != KERNEL_GATHER && BC != 4 && wide::g_wide2d) return 1;
-  if (g.ndim == 1 && kernel_kind != KERNEL_GATHER && BC != 4 && wide::g_seg1d) return 1;
   if (mixed_point_path(g, method, BC, kernel_kind)) return 1;
   if (!wide_path(g, BC, kernel_kind)) return method == 2 && has_dsc ? 2 : 1;  // (D,) F
   return method == 2 ? 3 : 2;  // (ghosts,) interior, faces

@@ -932,6 +932,8 @@ extern "C" int nlse_solver_stream(nlse_solver* s, void** stream) {
 
 extern "C" int nlse_solver_launches_per_step(const nlse_solver* s) {
   if (!s) return 0;
+  // whole steps per launch: a launch a step at most, counted as one a stage
+  if (step1d_shape(s->g, s->prob.method, s->prob.precision, s->kernel_kind).steps) return 4;
   if (s->prob.precision != NLSE_PREC_MIXED)
     return 4 * exact_stage_launches(s->g, s->prob.method, s->prob.bc, s->kernel_kind,
                                     s->prob.precision == NLSE_PREC_SINGLE, s->dsc != nullptr);
