@@ -20,7 +20,7 @@ cudaError_t launch_step2d_exact(const Geom& g, int BC, const Consts<float>& c, c
   switch (BC) {
     case 1: return by_shape<1>(g, c, in, V, out, shape, st);
     case 2: return by_shape<2>(g, c, in, V, out, shape, st);
-    case step2d::LARGE: return by_shape<3>(g, c, in, V, out, shape, st);
+    case 3: return by_shape<3>(g, c, in, V, out, shape, st);
   }
   return cudaErrorInvalidValue;
 }
