@@ -23,7 +23,8 @@ order) and ``wide.strips`` (1 by default: the 3D 2SHOC face kernels take the
 x faces' own lo, K and V from face-indexed arrays).
 
 Results are cached in a JSON file (``$NLSE_TUNE_CACHE`` or
-``~/.cache/nlse_gb300/tune.json``) keyed by device name and problem class;
+``~/.cache/nlse_gb300/tune.json``) keyed by device name, problem class and
+the meaning of the knobs (an entry of an older library is not used);
 :func:`apply` sets the knobs from the cache before a workload runs.  The
 knobs are process-wide and are read when a run starts: a solver whose graphs
 were captured under other values captures them again.
@@ -44,6 +45,10 @@ KNOBS = ("wide.zc", "wide.ty", "graph.steps", "wide2d.ty")
 # the library's own choice, timed beside the candidates (2D: a whole step per
 # launch, which no tile height of the stage kernels selects)
 DEFAULTS = {"wide.zc": 0, "wide.ty": 8, "graph.steps": 8, "wide2d.ty": 0}
+# Part of the cache's keys, raised when a knob's meaning or the kernels it
+# chooses between change: entries timed before are not used (2: a tile height
+# in wide2d.ty turns the whole-step kernels off)
+KNOB_SET = 2
 
 
 def set_knob(key, value):
@@ -72,8 +77,8 @@ def _device_name():
 
 def problem_key(shape, method, precision, BC):
     ndim, dims = grid_dims(shape)
-    return "%s|%dd|%s|m%d|p%d|bc%d" % (_device_name(), ndim, "x".join(str(d) for d in shape),
-                                       method, precision, BC)
+    return "k%d|%s|%dd|%s|m%d|p%d|bc%d" % (KNOB_SET, _device_name(), ndim,
+                                           "x".join(str(d) for d in shape), method, precision, BC)
 
 
 def _load_cache():

@@ -136,6 +136,26 @@ def test_stream_form_needs_no_d_scratch(lib):
         assert ng.Solver.bytes_for((300, 20), method=2, flags=flags, **args) == two
 
 
+def test_autotune_ignores_entries_of_other_knob_meanings(lib, tmp_path, monkeypatch):
+    # tuned when every 2D candidate was a launch per stage: 8 was the best tile
+    # height, and would now turn the whole-step kernels off
+    import json
+
+    from nlsemagic_gb300 import autotune
+    monkeypatch.setenv("NLSE_TUNE_CACHE", str(tmp_path / "tune.json"))
+    old = {"wide.zc": 0, "wide.ty": 8, "graph.steps": 10, "wide2d.ty": 8}
+    key = "%s|2d|256x256|m2|p3|bc1" % autotune._device_name()
+    (tmp_path / "tune.json").write_text(json.dumps({key: old}))
+    assert autotune.apply((256, 256), method=2, precision=3, BC=1) is None
+    assert autotune.get_knob("wide2d.ty") == 0
+    autotune._save_cache({autotune.problem_key((256, 256), 2, 3, 1): dict(old, **{"wide2d.ty": 0})})
+    saved = autotune.get_knob("graph.steps")
+    try:
+        assert autotune.apply((256, 256), method=2, precision=3, BC=1)["graph.steps"] == 10
+    finally:
+        autotune.set_knob("graph.steps", saved)
+
+
 def test_autotune_candidates_per_class():
     from nlsemagic_gb300 import autotune
     two = autotune.candidates((256, 256), 3)
