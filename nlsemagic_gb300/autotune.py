@@ -9,7 +9,8 @@ knobs and keeps the fastest:
                    CTA streams through; trades queue-fill overhead against the
                    number of CTAs in flight; 0: the library's choice),
 * ``wide.ty``      tile height of that kernel (4, 8 or 16 rows of 32 columns:
-                   halo re-reads against CTAs in flight),
+                   halo re-reads against CTAs in flight; neither is tried
+                   for grids that go by point, where they do not act),
 * ``graph.steps``  RK4 steps captured per CUDA graph (launch overhead against
                    graph size; matters for small grids),
 * ``wide2d.ty``    0: a whole step per launch where the library has it for
@@ -172,8 +173,11 @@ def tune(shape, method=2, precision=3, BC=2, steps=20, force=False, verbose=Fals
     saved = {k: get_knob(k) for k in KNOBS}
     results = []
     sv = _solver_for(shape, method, precision, BC)
+    cands = [dict(DEFAULTS)] + candidates(shape, precision)
+    if sv.ndim == 3 and sv.launches_per_step == 4:  # by point: wide.zc, wide.ty do not act
+        cands = [c for c in cands if c["wide.zc"] == 0 and c["wide.ty"] == 8]
     try:
-        for cfg in [dict(DEFAULTS)] + candidates(shape, precision):
+        for cfg in cands:
             t = time_config(shape, method, precision, BC, cfg, steps, solver=sv)
             results.append((t, cfg))
             if verbose:
