@@ -311,10 +311,11 @@ int nlse_take_steps_noalloc(const nlse_problem *p, const double *dUr, const doub
  *                  faces' own lo, K and V in face-indexed arrays that the
  *                  face kernel reads instead of the strided x faces; 0: the
  *                  full arrays.  Same bits.
- *   "small1d.max_points"  with "seg1d" 0, FP32 and mixed 1D solves of at
- *                  most this many points (default 2048, 0 = never, at most
- *                  65536) run each chunk in single-block launches instead of
- *                  a launch per pass.  Same bits.
+ *   "small1d.max_points"  FP32 and mixed 1D solves of at most this many
+ *                  points (default 2048, 0 = never, at most 65536) run each
+ *                  chunk in single-block launches: up to 128 or 256 points
+ *                  instead of the step kernel, with "seg1d" 0 instead of a
+ *                  launch per pass.  Same bits.
  *   "wide.z2"      1 (default): the mixed-precision 3D interior kernel (TMA
  *                  staging, both methods) advances two z planes per
  *                  iteration (one barrier and plane wait per two points);

@@ -84,11 +84,11 @@ static int g_default_graph_steps = 8;
 // the layout-conversion kernels in place, over the host link, instead of
 // being copied into a device staging buffer first.
 static int g_zero_copy = 1;
-// With the step kernel off ("seg1d" 0), FP32 and mixed 1D solves of at most
-// this many points run each chunk in single-block launches (0: never).  At
-// the 1024-point configuration this runs 2.0-2.6x faster than a launch per
-// pass; FP64 does not gain (one SM's FP64 rate is the limit there) and keeps
-// the stage launches.
+// FP32 and mixed 1D solves of at most this many points (0: none) run each chunk
+// in single-block launches, a thread per point, where the step kernel does not
+// take them (small1d_path) or is off ("seg1d" 0).  At the 1024-point
+// configuration this runs 2.0-2.6x faster than a launch per pass; FP64 does not
+// gain (one SM's FP64 rate is the limit there) and keeps the stage launches.
 static long long g_small1d_max = 2048;
 
 extern "C" int nlse_tune_set(const char* key, long long value) {
@@ -789,6 +789,18 @@ static int ensure_graph(nlse_solver* s, int parity) {
   return NLSE_OK;
 }
 
+// Whether a 1D solve runs in single-block launches rather than by the step
+// kernel, whose one warp takes four points a lane there.  Microseconds a step of
+// one solve alone, step kernel / single block: mixed CD MSD 64 points 2.7 / 2.2,
+// 128 2.6 / 2.2, 129 2.0 / 2.4 (several windows, and a launch for 10 steps);
+// mixed 2SHOC Dirichlet 64 3.4 / 2.3, 128 3.4 / 2.4, 256 2.8 / 2.6, 500 2.8 / 3.3,
+// MSD 128 4.8 / 3.8, 129 3.4 / 4.0; FP32 2SHOC Dirichlet 128 2.8 / 2.1, 200 2.3 / 2.5.
+static bool small1d_path(const nlse_solver* s) {
+  const nlse_problem& p = s->prob;
+  const bool slow_ends = p.method == 1 || p.bc == 2 || p.precision == NLSE_PREC_SINGLE;
+  return s->g.n <= (slow_ends ? 128 : 256);
+}
+
 // Small 1D solves: the whole chunk in single-block launches (at most 2^16
 // steps per launch, so that no launch runs for long).
 static int run_small1d(nlse_solver* s, long long nsteps) {
@@ -854,7 +866,9 @@ extern "C" int nlse_solver_run(nlse_solver* s, long long nsteps) {
   CUDA_TRY(cudaSetDevice(s->device));
   const Step1dShape sh =
       step1d_shape(s->g, s->prob.method, s->prob.precision, s->kernel_kind);
-  if (sh.steps) return run_step1d(s, sh, nsteps);
+  const bool small1d = s->g.ndim == 1 && s->g.n <= g_small1d_max &&
+                       s->prob.precision != NLSE_PREC_DOUBLE && (s->prob.method == 1 || s->dsc);
+  if (sh.steps && !(small1d && small1d_path(s))) return run_step1d(s, sh, nsteps);
   // Graphs of another form do not keep what the launches beside them rely on
   // (3D mixed: the x-face strips of lo, which steps by point leave behind)
   const unsigned form = g_form_changes;
@@ -863,9 +877,7 @@ extern "C" int nlse_solver_run(nlse_solver* s, long long nsteps) {
     free_graphs(s);
     s->form = form;
   }
-  if (s->g.ndim == 1 && s->g.n <= g_small1d_max && s->prob.precision != NLSE_PREC_DOUBLE &&
-      (s->prob.method == 1 || s->dsc) && nsteps > 0)
-    return run_small1d(s, nsteps);
+  if (small1d) return run_small1d(s, nsteps);
   // 3D 2SHOC mixed with x-face strips: filled (where stale) before the
   // steps, outside any graph
   int sr = 0;

@@ -1,0 +1,36 @@
+"""On both sides of the sizes where a solve changes its kernels: the bits of the
+gather kernels (contracted FP64: its rounding)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _state(shape):
+    X = np.meshgrid(*[0.2 * np.arange(n) for n in shape], indexing="ij")
+    U = (0.8 + 0.2 * np.cos(0.7 * X[0]) * np.cos(0.5 * X[-1])) * np.exp(0.3j * X[0] - 0.2j * X[-1])
+    return U, 0.1 * np.cos(0.4 * X[0] + 0.3 * X[-1])
+
+
+def _run(shape, method, prec, BC, flags=0, runs=(11,)):
+    import nlsemagic_gb300 as ng
+    U, V = _state(shape)
+    with ng.Solver(shape, method=method, precision=prec, BC=BC, s=-1.0, a=1.0, h2=0.04, k=0.004,
+                   flags=ng.FLAG_MSD_GUARD | flags) as sv:
+        sv.upload(U, V)
+        for n in runs:
+            sv.run(n)
+        return np.ascontiguousarray(sv.download()).view(np.float64)
+
+
+@pytest.mark.parametrize("prec", [1, 3])
+@pytest.mark.parametrize("method", [1, 2])
+@pytest.mark.parametrize("BC", [1, 2, 3, 4])
+def test_small_1d(gpu_lib, BC, method, prec):
+    # single-block launches up to 128 or 256 points, the step kernel above
+    import nlsemagic_gb300 as ng
+    for n in (4, 127, 128, 129, 255, 256, 257):
+        want = _run((n,), method, prec, BC, ng.FLAG_GATHER)
+        assert np.all(np.isfinite(want))
+        assert np.array_equal(_run((n,), method, prec, BC), want), n
+        assert np.array_equal(_run((n,), method, prec, BC, runs=(1, 3, 7)), want), n
