@@ -43,8 +43,11 @@ __global__ void __launch_bounds__(NT)
   constexpr int DX = METHOD == 2 ? TX + 2 : 1, DY = METHOD == 2 ? TY + 2 : 1;
   __shared__ __align__(16) C2<R> su[SY][SX];  // cp.async destinations: 8/16-byte aligned
   __shared__ C2<R> sd[DY][DX];                 // 2SHOC: D on the tile and a 1-cell halo
-  // (no early trigger of the next launch: its blocks would be placed while these
-  // come and go; 2SHOC 300^2 16.9 -> 12.9 us a step)
+  // The next launch is triggered at the start where this one is a few blocks and
+  // waits for nothing but latency (CD 8 x 8 6.2 us a step, 5.1 so; 2SHOC 17 x 18
+  // 10.1, 9.5); not where its blocks would be placed while these come and go
+  // (2SHOC 300^2, 380 blocks, 12.2 without and 14.8 so; 181^2, 138 blocks, 11.2, 11.6).
+  if (gridDim.x * gridDim.y <= 8) pdl_trigger();
   pdl_wait();  // the previous kernel's output
   const int M = g.M, N = g.N;
   // one CTA per tile: a two-dimensional grid, or (nbx > 0: more tile rows

@@ -34,3 +34,15 @@ def test_small_1d(gpu_lib, BC, method, prec):
         assert np.all(np.isfinite(want))
         assert np.array_equal(_run((n,), method, prec, BC), want), n
         assert np.array_equal(_run((n,), method, prec, BC, runs=(1, 3, 7)), want), n
+
+
+@pytest.mark.parametrize("method", [1, 2])
+@pytest.mark.parametrize("BC", [1, 2, 3])
+def test_fp32_2d_few_blocks(gpu_lib, BC, method):
+    # the next launch triggered early up to 8 blocks (32 x 8 tiles): races would
+    # show in repeated runs
+    import nlsemagic_gb300 as ng
+    for shape in [(3, 3), (9, 8), (15, 15), (32, 64), (33, 64), (64, 33), (15, 130), (300, 9)]:
+        want = _run(shape, method, 1, BC, ng.FLAG_GATHER, (41,))
+        for _ in range(3):
+            assert np.array_equal(_run(shape, method, 1, BC, runs=(41,)), want), shape
