@@ -32,6 +32,25 @@ static bool point_path(const Geom& g, int method, int BC, int kernel_kind, bool 
   return !single || (method == 2 || BC == 2 || g.M % 2 || g.n <= (1LL << 20));
 }
 
+// Where one point's chain of dependent instructions is all the time there is: by
+// point, a thread next to a face does that face's points after its own, up to
+// seven of them at a corner; by gather each has its thread.  Microseconds a step
+// of one solve alone / of three in flight, by point -> by gather:
+//   FP64 2D CD    Dirichlet 8^2 13.6 / 6.0 -> 9.1 / 3.4    48^2 15.4 / 5.8 -> 14.8 / 5.6
+//                 64^2 13.9 / 5.5 against 15.1 / 6.2
+//                 MSD  8^2 17.8 / 7.2 -> 15.7 / 6.2  12^2 18.5 / 7.2 against 19.2 / 7.1
+//           2SHOC Dirichlet 8^2 27.5 / 11.1 -> 20.2 / 7.5  18^2 30.0 / 11.2 -> 29.8 / 10.4
+//                 24^2 29.0 / 10.9 against 30.8 / 10.7
+//                 MSD 10^2 35.4 / 12.7 -> 33.0 / 11.5  12^2 34.6 / 12.8 against 40.4 / 14.2
+//   3D (the streaming kernels, which 3D had before, in the middle), MSD 2SHOC
+//                 FP64 3^3 80.0 / 52.2 / 40.4   FP32 3^3 25.6 / 24.2 / 14.0
+bool gather_small(const Geom& g, int method, int BC, int kernel_kind, bool single) {
+  if (kernel_kind != KERNEL_TILED || BC > 3) return false;
+  if (g.ndim == 3) return g.n <= 64;
+  if (g.ndim != 2 || single) return false;
+  return g.n <= (BC == 2 ? 128 : (method == 1 ? 3 << 10 : 5 << 6));
+}
+
 // D scratch: 2SHOC in gather form and by point.  FP32 2D grids on the tile
 // kernel take none; should the knob turn it off later, the gather kernel
 // recomputes D.  The contracted class takes the wide form by point, without D
@@ -39,7 +58,8 @@ static bool point_path(const Geom& g, int method, int BC, int kernel_kind, bool 
 long long exact_dsc_entries(const Geom& g, int method, int BC, int kernel_kind, bool single,
                             bool contracted) {
   if (method != 2) return 0;
-  if (contracted && g.ndim >= 2 && kernel_kind != KERNEL_GATHER) return 0;
+  if (contracted && g.ndim >= 2 && kernel_kind != KERNEL_GATHER)
+    return gather_small(g, method, BC, kernel_kind, false) ? g.n : 0;
   if (g.ndim == 3 && kernel_kind == KERNEL_STREAM) return 0;
   return tile2d_path(g, method, BC, kernel_kind, single) ? 0 : g.n;
 }
@@ -63,6 +83,7 @@ template <typename R>
 cudaError_t launch_exact_stage(const Geom& g, int method, int BC, const Consts<R>& c,
                                const ExactStageArgs<R>& a, int stage, cudaStream_t st,
                                int kernel_kind) {
+  if (gather_small(g, method, BC, kernel_kind, sizeof(R) == 4)) kernel_kind = KERNEL_GATHER;
   // (2SHOC whose D scratch did not fit forms D on the way)
   if (point_path(g, method, BC, kernel_kind, sizeof(R) == 4) && (method == 1 || a.dsc))
     return launch_point_exact<R>(g, method, BC, c, a, stage, st);

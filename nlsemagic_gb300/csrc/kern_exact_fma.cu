@@ -12,6 +12,7 @@ namespace nlse {
 cudaError_t launch_exact_stage_fma(const Geom& g, int method, int BC, const Consts<double>& c,
                                    const ExactStageArgs<double>& a, int stage, cudaStream_t st,
                                    int kernel_kind) {
+  if (gather_small(g, method, BC, kernel_kind, false)) kernel_kind = KERNEL_GATHER;
   if (g.ndim >= 2 && BC <= 3 && kernel_kind != KERNEL_GATHER)
     return launch_point_fma(g, method, BC, c, a, stage, st);
   return launch_exact_stage_var<double, 1>(g, method, BC, c, a, stage, st, kernel_kind);

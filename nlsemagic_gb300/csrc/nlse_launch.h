@@ -68,6 +68,10 @@ cudaError_t launch_exact_stage_fma(const Geom& g, int method, int BC, const Cons
                                    const ExactStageArgs<double>& a, int stage, cudaStream_t st,
                                    int kernel_kind);
 
+// Whether a grid is so small that its FP64 (2D, 3D) or FP32 (3D) stages run by
+// gather, not by point (kern_exact.cu).
+bool gather_small(const Geom& g, int method, int BC, int kernel_kind, bool single);
+
 // Thread-per-point stages in 2D and 3D (kern_point.cuh): exact, contracted.
 template <typename R>
 cudaError_t launch_point_exact(const Geom& g, int method, int BC, const Consts<R>& c,
