@@ -36,6 +36,25 @@ namespace step2d {
 
 enum { SMALL = 1, MIDDLE = 2, LARGE = 3 };  // step2d_shape
 
+// What a step of a grid costs in tiles of tx x ty cells, `cells` evaluated in
+// stage 1, in cells of an inner tile: a tile at a face runs the tests of every
+// cell and, with MSD, waits for a quotient twice a stage; where the face is one
+// lane of each warp (x) more than where it is whole rows (y).  Weights from
+// launches of such tiles only (sides of 16 to 128 points by up to 62500).
+inline double step_cells(const Geom& g, int BC, int tx, int ty, int cells) {
+  const double nbx = (g.M + tx - 1) / tx, nby = (g.N + ty - 1) / ty;
+  const double ix = nbx > 2 ? nbx - 2 : 0, iy = nby > 2 ? nby - 2 : 0;
+  const double wx = BC == 2 ? 2.6 : 1.65, wy = BC == 2 ? 1.8 : 1.5;
+  return cells * ((nbx - ix) * nby * wx + ix * (nby - iy) * wy + ix * iy);
+}
+// The stage launches' share: a stage of a step in the cells of their tiles, over
+// the cost of an inner tile's cell.
+inline double stage_cells(const Geom& g, int method, bool single) {
+  const double ratio = method == 2 ? 0.30 : (single ? 0.22 : 0.27);
+  const int ty = wide2d::pick_ty(g);
+  return (double)wide2d::tiles(g, ty) * 32 * ty / ratio;
+}
+
 // XT x G threads of R rows: the cells stage 1 is evaluated on.
 template <int METHOD, int XT, int G, int R>
 struct Shape {

@@ -56,17 +56,41 @@ static cudaError_t by_shape(const Geom& g, const Consts<float>& c, const float2*
 // launch's come and go and load the SMs unevenly (300^2 CD three in flight 2.6,
 // 2.3 so).
 // A grid of fewer than 16 points a side fills too little of a tile (8000 x 8:
-// 3.8 against 5.4 with three in flight).
+// 3.8 against 5.4 with three in flight), and where most tiles are at a face and
+// more than can all start at once, the stage launches, whose faces cost less, are
+// the faster form: by step_cells.  Stage launches, this: 2SHOC MSD 16 x 62500 89 /
+// 81, 161 / 158; 64 x 15625 49 / 42, 95 / 91; 15625 x 64 39 / 32, 39 / 35; 128 x 7812
+// 46 / 36, 62 / 52; 64 x 1406 16 / 5.8, 12 / 10; CD MSD 32 x 31250 39 / 32, 60 / 56,
+// 15625 x 64 31 / 25, 25 / 20; FP32 CD MSD 64 x 15625 32 / 27, 44 / 41.  Of 432
+// narrow grids of 2e4 to 1e6 points the rule takes the slower form by more than
+// 5% (mean of both figures) on 3.
+// Mixed CD MSD up to 2^11 points: 24^2 6.9 / 2.6 stage launches, 7.7 / 2.8 so.
 int step2d_shape(const Geom& g, int method, int BC, int precision, int kernel_kind) {
   using namespace step2d;
   if (g.ndim != 2 || kernel_kind == KERNEL_GATHER || !wide::g_wide2d || wide2d::g_ty) return 0;
   if (precision == 2 || (precision == 1 && method == 2) || BC > 3) return 0;
   if (g.M < 16 || g.N < 16 || g.N > 65535 * 20) return 0;  // tile rows: gridDim.y
-  if (precision == 1) return g.n <= (1LL << 19) ? SMALL : LARGE;
-  if (method == 1) return g.n <= (1LL << 18) ? SMALL : (g.n <= (1LL << 20) ? MIDDLE : LARGE);
-  if (g.n <= (1LL << 15)) return MIDDLE;
-  if (g.n <= (1LL << 17)) return SMALL;
-  return BC == 2 && g.n <= (1LL << 18) ? MIDDLE : LARGE;
+  const bool cd = method == 1, single = precision == 1;
+  if (cd && !single && BC == 2 && g.n <= (1LL << 11)) return 0;
+  int shape = LARGE;
+  if (single)
+    shape = g.n <= (1LL << 19) ? SMALL : LARGE;
+  else if (cd)
+    shape = g.n <= (1LL << 18) ? SMALL : (g.n <= (1LL << 20) ? MIDDLE : LARGE);
+  else if (g.n <= (1LL << 15) || (BC == 2 && g.n > (1LL << 17) && g.n <= (1LL << 18)))
+    shape = MIDDLE;
+  else if (g.n <= (1LL << 17))
+    shape = SMALL;
+  // the tiles of by_shape; so few all start at once
+  const bool wide = cd ? shape == LARGE : shape != MIDDLE;
+  const int tx = cd ? (wide ? 58 : 26) : (wide ? 52 : 20), ty = cd ? 26 : 20;
+  const int nbx = (g.M + tx - 1) / tx;
+  const long long tiles = (long long)nbx * ((g.N + ty - 1) / ty);
+  int at_once = !cd && shape == SMALL ? 152 : 280;
+  if (BC == 2 && nbx <= 2) at_once /= 2;  // none away from an x face
+  if (tiles > at_once && step_cells(g, BC, tx, ty, wide ? 2048 : 1024) > stage_cells(g, method, single))
+    return 0;
+  return shape;
 }
 
 cudaError_t launch_step2d_mixed(const Geom& g, int method, int BC, const Consts<float>& c,

@@ -66,3 +66,22 @@ def test_small_grids_by_gather(gpu_lib, BC, method, flags):
             assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want), shape
         else:
             assert np.array_equal(got, want), shape
+
+
+@pytest.mark.parametrize("prec,method", [(3, 1), (3, 2), (1, 1)])
+@pytest.mark.parametrize("BC", [1, 2, 3])
+def test_narrow_2d(gpu_lib, BC, prec, method):
+    # whole steps or stage launches by the share of tiles at a face: the bits of
+    # the stage launches ("wide2d.ty" 16)
+    from nlsemagic_gb300 import autotune
+    old = autotune.get_knob("wide2d.ty")
+    for shape in [(16, 9000), (9000, 17), (64, 3000), (3001, 63), (128, 1600), (27, 5400), (24, 24),
+                  (45, 45), (46, 45), (530, 531)]:
+        got = _run(shape, method, prec, BC, runs=(9, 2))
+        try:
+            autotune.set_knob("wide2d.ty", 16)
+            want = _run(shape, method, prec, BC, runs=(11,))
+        finally:
+            autotune.set_knob("wide2d.ty", old)
+        assert np.all(np.isfinite(want))
+        assert np.array_equal(got, want), shape
