@@ -215,9 +215,9 @@ long long nlse_solver_bytes_for(const nlse_problem *p);
  * in one persistent launch per precision class and call of nlse_batch_run,
  * driven by a tile work queue: mixed 1D and 2D solves in whole RK4 steps
  * ordered per solve; everything else (and a run whose mixed solves include a
- * 3D one) one pass over all tiles per RK4 stage, separated by a bounded grid
- * barrier.  State lives in a device pool of a fixed byte
- * budget; solves are admitted while the pool has room and keep their state
+ * 3D one, or are mostly narrow 2D grids) one pass over all tiles per RK4 stage,
+ * separated by a bounded grid barrier.  State lives in a device pool of a fixed
+ * byte budget; solves are admitted while the pool has room and keep their state
  * resident until removed.  No reference counterpart (the reference runs one
  * solve per MEX call).
  * ---------------------------------------------------------------------- */

@@ -2,7 +2,7 @@
 // include/nlse_gb300.h).
 //
 // Device side: a run whose mixed solves are all 1D or 2D takes them in whole RK4
-// steps (nlse_batch_steps.cu).  Everything else (batch_kern.cuh): a cooperative
+// steps (nlse_batch_steps.cu), unless narrow 2D grids prevail.  Everything else (batch_kern.cuh): a cooperative
 // persistent kernel.  All active solves are cut
 // into tiles; per RK4 stage every CTA pulls tiles from an atomic work-queue
 // counter of that stage until the queue is empty, evaluates the stage on the
@@ -43,6 +43,9 @@ int set_error(int code, const char* fmt, ...);
 bool batch_steps_takes(const nlse_problem& p);
 long long batch_steps_tiles(const void* solve);
 long long batch_steps_rounds(const void* solve, long long adv);
+double batch_steps_time(const void* solve);
+double batch_stages_time(const void* solve);
+double batch_barriers_time();
 cudaError_t batch_steps_launch(const void* solves, const void* tiles, int ntiles,
                                const int* tile_n, int max_steps, long long rounds,
                                unsigned long long* queue, int* err, long long budget, int sms,
@@ -99,8 +102,9 @@ struct nlse_batch {
   unsigned long long* d_queue = nullptr;
   int *d_tile_n = nullptr, *h_tile_n = nullptr;
   int sms = 0;
-  // resident CTAs: FP64, mixed, contracted FP64
-  int max_blocks[3] = {0, 0, 0};
+  // resident CTAs: FP64, mixed, mixed in segment / rectangle tiles only,
+  // contracted FP64
+  int max_blocks[4] = {0, 0, 0, 0};
   int last_launches = 0;
 };
 
@@ -211,16 +215,21 @@ extern "C" int nlse_batch_create(long long pool_bytes, int max_solves, nlse_batc
   }
   cudaMemsetAsync(b->d_bar, 0, sizeof(BarrierState), b->stream);
   cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream);
-  int per64 = 0, permx = 0;
+  int per64 = 0, permx = 0, perst = 0;
   cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per64, batch_kernel<NLSE_PREC_DOUBLE>, BT, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&permx, batch_kernel<NLSE_PREC_MIXED>, BT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per64, batch_kernel<NLSE_PREC_DOUBLE, false>,
+                                                BT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&permx, batch_kernel<NLSE_PREC_MIXED, false>,
+                                                BT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perst, batch_kernel<NLSE_PREC_MIXED, true>,
+                                                BT, 0);
   const int perfma = nlse::batch_fma_blocks_per_sm();
-  if (per64 < 1 || permx < 1 || perfma < 1)
+  if (per64 < 1 || permx < 1 || perst < 1 || perfma < 1)
     return cleanup(nlse::set_error(NLSE_ERR_CUDA, "batch kernel cannot be resident"));
   b->max_blocks[0] = b->sms * per64;
   b->max_blocks[1] = b->sms * permx;
-  b->max_blocks[2] = b->sms * perfma;
+  b->max_blocks[2] = b->sms * perst;
+  b->max_blocks[3] = b->sms * perfma;
   *out = b;
   return NLSE_OK;
 }
@@ -338,11 +347,18 @@ extern "C" int nlse_batch_run(nlse_batch* b, int max_steps) {
   std::vector<int> which[NC];
   long long ntiles[NC] = {0, 0, 0}, ntiles_d[NC] = {0, 0, 0};
   int steps[NC] = {0, 0, 0};
-  // mixed 1D and 2D solves alone: whole steps per task (nlse_batch_steps.cu)
+  // mixed 1D and 2D solves alone: whole steps per task (nlse_batch_steps.cu), but
+  // where most of the work is on narrow 2D grids, whose tiles are all at a face
   bool stepwise = true;
+  double by_steps = 0, by_stages = 0;
   for (const Slot& S : b->slots)
-    if (S.used && S.d.steps_left > 0 && S.d.prec != NLSE_PREC_DOUBLE)
+    if (S.used && S.d.steps_left > 0 && S.d.prec != NLSE_PREC_DOUBLE) {
       stepwise = stepwise && nlse::batch_steps_takes(S.prob);
+      if (!stepwise) break;
+      by_steps += nlse::batch_steps_time(&S.d);
+      by_stages += nlse::batch_stages_time(&S.d);
+    }
+  if (by_steps > by_stages + nlse::batch_barriers_time()) stepwise = false;
   auto count = [&](const BSolve& d) {
     return stepwise && d.prec != NLSE_PREC_DOUBLE ? nlse::batch_steps_tiles(&d) : tile_count(d);
   };
@@ -429,7 +445,9 @@ extern "C" int nlse_batch_run(nlse_batch* b, int max_steps) {
     const size_t np = (size_t)steps[c] * 8;
     BTRY(cudaMemsetAsync(b->d_qctr, 0, sizeof(unsigned) * np, b->stream));
     BTRY(cudaMemsetAsync(b->d_bar, 0, sizeof(BarrierState), b->stream));
-    int blocks = b->max_blocks[c];
+    bool staged = c == 1;  // every solve of the class in segment / rectangle tiles
+    for (int id : which[c]) staged = staged && tile_kind(b->slots[id].d) != K_LINEAR;
+    int blocks = b->max_blocks[c == 2 ? 3 : staged ? 2 : c];
     if ((long long)blocks > ntiles[c]) blocks = (int)ntiles[c];
     const BTile* tiles = b->d_tiles + first;
     int nt_i = (int)ntiles[c], ntd_i = (int)ntiles_d[c], st_i = steps[c];
@@ -438,8 +456,9 @@ extern "C" int nlse_batch_run(nlse_batch* b, int max_steps) {
     if (c == 2) {
       BTRY(nlse::batch_fma_launch((unsigned)blocks, args, b->stream));
     } else {
-      const void* kern = c == 0 ? (const void*)batch_kernel<NLSE_PREC_DOUBLE>
-                                : (const void*)batch_kernel<NLSE_PREC_MIXED>;
+      const void* kern = c == 0   ? (const void*)batch_kernel<NLSE_PREC_DOUBLE, false>
+                         : staged ? (const void*)batch_kernel<NLSE_PREC_MIXED, true>
+                                  : (const void*)batch_kernel<NLSE_PREC_MIXED, false>;
       BTRY(cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(BT), args, 0, b->stream));
     }
     ++b->last_launches;

@@ -8,7 +8,7 @@ namespace nlse {
 
 int batch_fma_blocks_per_sm() {
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<NLSE_PREC_DOUBLE>, BT,
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<NLSE_PREC_DOUBLE, false>, BT,
                                                     0) != cudaSuccess)
     return 0;
   return n;
@@ -16,7 +16,7 @@ int batch_fma_blocks_per_sm() {
 
 // args: those of batch_kernel, as cudaLaunchCooperativeKernel takes them
 cudaError_t batch_fma_launch(unsigned blocks, void** args, cudaStream_t st) {
-  return cudaLaunchCooperativeKernel((const void*)batch_kernel<NLSE_PREC_DOUBLE>,
+  return cudaLaunchCooperativeKernel((const void*)batch_kernel<NLSE_PREC_DOUBLE, false>,
                                      dim3(blocks), dim3(BT), args, 0, st);
 }
 

@@ -178,6 +178,31 @@ long long batch_steps_tiles(const void* solve) {
   const step1d::Plan pl = step1d::make_plan(d.g.n, d.method, R1, round_steps(d), WARPS1);
   return pl.blocks;
 }
+// Estimated time of a step of a solve, nanoseconds of the whole chip, in this launch
+// and by stage passes on segments and rectangles (batch_kern.cuh), whose four grid
+// barriers cost batch_barriers_time whatever the solves.  Measured and (estimated),
+// microseconds a step of 24 solves, by stage passes / here:
+//   8 x 8000 MSD    CD 262 (274) / 353 (394)   2SHOC 314 (328) / 580 (665)
+//   3 x 9000        CD 211 (230) / 286 (281)   2SHOC 248 (277) / 475 (474)
+//   64 x 1500 MSD   CD 121 (128) / 152 (148)   2SHOC 153 (148) / 240 (249)
+//   128 x 700 MSD   CD 112 (122) /  91 (88)    2SHOC 139 (141) / 143 (140)
+//   300 x 300 MSD   CD 114 (134) /  69 (57)    2SHOC 133 (155) / 103 (92)
+double batch_steps_time(const void* solve) {
+  const BSolve& d = *(const BSolve*)solve;
+  const bool cd = d.method == 1;
+  if (d.g.ndim == 1) return d.g.n * (cd ? 6e-3 : 9e-3);
+  return step2d::step_cells(d.g, d.bc, cd ? Shape1::TX : Shape2::TX, cd ? Shape1::TY : Shape2::TY,
+                            XT * GT * RT) *
+         (cd ? 10e-3 : 13e-3);
+}
+double batch_stages_time(const void* solve) {
+  const BSolve& d = *(const BSolve*)solve;
+  const bool cd = d.method == 1;
+  if (d.g.ndim == 1) return d.g.n * 28e-3;
+  return wide2d::tiles(d.g, W2_TY) * (d.bc == 2 ? (cd ? 39.0 : 48.0) : (cd ? 28.0 : 35.0));
+}
+double batch_barriers_time() { return 40000.0; }
+
 long long batch_steps_rounds(const void* solve, long long adv) {
   const int per = round_steps(*(const BSolve*)solve);
   return (adv + per - 1) / per;
