@@ -40,7 +40,8 @@ static bool point_path(const Geom& g, int method, int BC, int kernel_kind, bool 
 //                 64^2 13.9 / 5.5 against 15.1 / 6.2
 //                 MSD  8^2 17.8 / 7.2 -> 15.7 / 6.2  12^2 18.5 / 7.2 against 19.2 / 7.1
 //           2SHOC Dirichlet 8^2 27.5 / 11.1 -> 20.2 / 7.5  18^2 30.0 / 11.2 -> 29.8 / 10.4
-//                 24^2 29.0 / 10.9 against 30.8 / 10.7
+//                 24^2 29.0 / 10.9 against 30.8 / 10.7; LAP0 15^2 28.0 / 10.0 against
+//                 28.7 / 10.1
 //                 MSD 10^2 35.4 / 12.7 -> 33.0 / 11.5  12^2 34.6 / 12.8 against 40.4 / 14.2
 //   3D (the streaming kernels, which 3D had before, in the middle), MSD 2SHOC
 //                 FP64 3^3 80.0 / 52.2 / 40.4   FP32 3^3 25.6 / 24.2 / 14.0
@@ -48,7 +49,7 @@ bool gather_small(const Geom& g, int method, int BC, int kernel_kind, bool singl
   if (kernel_kind != KERNEL_TILED || BC > 3) return false;
   if (g.ndim == 3) return g.n <= 64;
   if (g.ndim != 2 || single) return false;
-  return g.n <= (BC == 2 ? 128 : (method == 1 ? 3 << 10 : 5 << 6));
+  return g.n <= (BC == 2 ? 128 : (method == 1 ? 3 << 10 : (BC == 1 ? 320 : 240)));
 }
 
 // D scratch: 2SHOC in gather form and by point.  FP32 2D grids on the tile

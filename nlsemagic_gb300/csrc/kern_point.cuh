@@ -236,9 +236,9 @@ __global__ void __launch_bounds__(NT)
   }
   T2 Fq;
   if (FORM == WIDE) {
-    T2 t1 = {0, 0}, s2 = {0, 0};
+    T2 t1 = second(Yin[p + 1], yq, Yin[p - 1]), s2;
 #pragma unroll
-    for (int a = 0; a < DIM; ++a)
+    for (int a = 1; a < DIM; ++a)
       t1 = add(t1, second(Yin[p + s[a]], yq, Yin[p - s[a]]));
     const T2 dq = {c.lh2 * t1.r, c.lh2 * t1.i};
 #pragma unroll
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(NT)
             if (e != a) st = add(st, second(Yin[b + s[e]], yb, Yin[b - s[e]]));
           far = axpy(axpy(yb, (R)-1, st), c.h2, db);
         }
-        s2 = add(s2, far);
+        s2 = a == 0 && d < 0 ? far : add(s2, far);
       }
     Fq = rhs_wide<R, DIM>(c, yq, vq, t1, s2);
   } else {

@@ -33,7 +33,8 @@ using wide2d::BY;
 using wide2d::NT;
 using wide2d::TX;
 
-template <typename R, int METHOD, int BC, int TY>
+// EARLY: a launch of few blocks (launch_ty)
+template <typename R, int METHOD, int BC, int TY, bool EARLY>
 __global__ void __launch_bounds__(NT)
     exact2d(Geom g, Consts<R> c, const C2<R>* __restrict__ Yin, C2<R>* Psi,
             const R* __restrict__ V, C2<R>* __restrict__ K, C2<R>* __restrict__ Yout, int stage,
@@ -46,8 +47,9 @@ __global__ void __launch_bounds__(NT)
   // The next launch is triggered at the start where this one is a few blocks and
   // waits for nothing but latency (CD 8 x 8 6.2 us a step, 5.1 so; 2SHOC 17 x 18
   // 10.1, 9.5); not where its blocks would be placed while these come and go
-  // (2SHOC 300^2, 380 blocks, 12.2 without and 14.8 so; 181^2, 138 blocks, 11.2, 11.6).
-  if (gridDim.x * gridDim.y <= 8) pdl_trigger();
+  // (2SHOC 300^2, 380 blocks, 12.2 without and 14.8 so; 181^2, 138 blocks, 11.2,
+  // 11.6).  A test of the grid here costs every size 1.5%.
+  if (EARLY) pdl_trigger();
   pdl_wait();  // the previous kernel's output
   const int M = g.M, N = g.N;
   // one CTA per tile: a two-dimensional grid, or (nbx > 0: more tile rows
@@ -144,8 +146,11 @@ cudaError_t launch_ty(const Geom& g, const Consts<R>& c, const ExactStageArgs<R>
   const bool flat = nby > 65535;
   const dim3 grid(flat ? (unsigned)wide2d::tiles(g, TY) : (unsigned)nbx, flat ? 1u : (unsigned)nby);
   const dim3 block(BX, BY);
-  return launch_k(exact2d<R, METHOD, BC, TY>, grid, block, 0, st, pdl, g, c, a.Yin, a.Psi, a.V,
-                  a.K, a.Yout, stage, sx, sy, flat ? nbx : 0);
+  auto k = exact2d<R, METHOD, BC, TY, false>;
+  if constexpr (TY == 8)  // what a grid of few tiles takes
+    if (nbx * nby <= 8) k = exact2d<R, METHOD, BC, TY, true>;
+  return launch_k(k, grid, block, 0, st, pdl, g, c, a.Yin, a.Psi, a.V, a.K, a.Yout, stage, sx, sy,
+                  flat ? nbx : 0);
 }
 
 template <typename R, int METHOD, int BC>

@@ -52,12 +52,12 @@ def test_fp32_2d_few_blocks(gpu_lib, BC, method):
 @pytest.mark.parametrize("method", [1, 2])
 @pytest.mark.parametrize("BC", [1, 2, 3])
 def test_small_grids_by_gather(gpu_lib, BC, method, flags):
-    # 2D FP64: 128 points (MSD), 3072 (CD) or 320 (2SHOC); 3D: 64
+    # 2D FP64: 128 points (MSD), 3072 (CD) or 320 and 240 (2SHOC); 3D: 64
     import nlsemagic_gb300 as ng
     prec, f = {"fp32": (1, 0), "fp64": (2, 0), "contracted": (2, ng.FLAG_FMA)}[flags]
     shapes = [(3, 3, 3), (4, 4, 4), (3, 3, 8), (5, 13, 3), (4, 4, 5)]
     if prec == 2:
-        shapes += [(3, 3), (16, 8), (43, 3), (16, 20), (107, 3), (48, 64), (439, 7), (3, 1200)]
+        shapes += [(3, 3), (16, 8), (43, 3), (15, 16), (16, 20), (107, 3), (48, 64), (439, 7), (3, 1200)]
     for shape in shapes:
         got = _run(shape, method, prec, BC, f, (9, 1))
         want = _run(shape, method, prec, BC, f | ng.FLAG_GATHER, (10,))
