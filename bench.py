@@ -48,13 +48,15 @@ UNIT = "Gpt-steps/s"
 BYTES_MODEL_MIXED = 240.0
 BYTES_DESIGN_MIXED = 160.0
 BYTES_FP64 = 304.0
-# FP64 instructions per interior grid-point-step of the exact FP64 class,
-# counted from the reference expressions (each +, -, x one instruction; the
-# reference operation order forbids contraction): 3D 2SHOC per stage D 16,
-# F 57 (the |U|^2 term shared by both components), update 7 -> 80 x 4; 2D
-# 2SHOC D 12, F 35, update 7 -> 54 x 4 (src/NLSEmagic3D/NLSE3D_TAKE_STEPS_2SHOC.c:
-# 56-72, 233-262; src_old/NLSE2D_v1/NLSE2D_TAKE_STEPS_2SHOC.c:59-67, 169-187).
-FP64_OPS = {(3, 2): 320.0, (2, 2): 216.0}
+# FP64 instructions per interior grid-point-step of the exact FP64 class.  2D
+# 2SHOC: counted from the reference expressions (each +, -, x one instruction; the
+# reference operation order forbids contraction), per stage D 12, F 35, update 7
+# -> 54 x 4 (src_old/NLSE2D_v1/NLSE2D_TAKE_STEPS_2SHOC.c:59-67, 169-187).  3D 2SHOC:
+# the expressions have 80 x 4 (src/NLSEmagic3D/NLSE3D_TAKE_STEPS_2SHOC.c:56-72,
+# 233-262), of which the kernels issue 307, the common ones once (ncu's FP64 pipe
+# count at 160^3, 16.8 for D and 57.6 to 61.7 for F and the update a stage, less the
+# boundary's share).
+FP64_OPS = {(3, 2): 307.0, (2, 2): 216.0}
 # The timed CPU arm is the C restatement of the reference integrator (the
 # reference's own build cannot travel to an aarch64 host).  Both were timed
 # side by side on one x86-64 core (320^3, one RK4 step of FP64 2SHOC MSD, the

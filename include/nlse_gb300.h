@@ -290,16 +290,17 @@ int nlse_take_steps_noalloc(const nlse_problem *p, const double *dUr, const doub
 
 /* ------------------------------------------------------------------------
  * Launch tuning knobs (process-wide; no reference counterpart; set by the
- * autotuner in nlsemagic_gb300/autotune.py).  They are read when a stage
- * launch is issued or a CUDA graph captured, so they affect solvers created
- * (or graphs captured) afterwards.  Keys:
+ * autotuner in nlsemagic_gb300/autotune.py).  They act on every run that
+ * starts afterwards: graphs captured under other values are captured again
+ * ("graph.steps": on solvers created afterwards).  Keys:
  *   "wide.zc"      z-chunk length of the mixed-precision 3D kernel (planes a
  *                  CTA streams through); 0 = built-in heuristic.
  *   "graph.steps"  RK4 steps per captured graph for new solvers (default 8).
  *   The wide.* knobs choose between forms of the mixed-precision 3D streaming
  *   kernels.  Small 3D grids, and grids with an odd number of points a row,
  *   run by point instead (one launch per stage, same bits) while "wide.pdl",
- *   "wide.strips", "wide.z2" and "wide.tile_order" are all 1.
+ *   "wide.strips", "wide.z2" and "wide.tile_order" are all 1 and the problem
+ *   does not have NLSE_FLAG_STREAM.
  *   "wide.pdl"     1 (default): the mixed-precision 3D 2SHOC stage kernels
  *                  (face ghosts, interior, faces) are launched with
  *                  programmatic dependent launch, so a stage's interior

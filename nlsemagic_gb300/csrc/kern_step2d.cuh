@@ -19,10 +19,9 @@
 // beyond a face point is its hi (constant) and an E that each stage writes
 // into the E plane's cell beyond the face before it is read.
 //
-// What bounds it: shared-memory reads and FP32 latency (2048^2 2SHOC: about 36 B
-// of HBM traffic per point and step against 160 B of the stage launches; LDS
-// wavefronts at half their rate, 2.2 instructions a clock); what both took is
-// beside step2d_shape.
+// What bounds it: shared-memory reads and FP32 latency (2048^2 2SHOC: 33 B of HBM
+// traffic per point and step against 160 B of the stage launches; shared memory at
+// 73% of its rate); what both took is beside step2d_shape.
 //
 // Tiles start at floor(i M / nbx), floor(j N / nby): sizes that differ by one
 // cell at most and are at least 2, so a face point and its MSD neighbour are

@@ -12,8 +12,8 @@
 namespace nlse {
 namespace wide {
 extern int g_pdl;     // stage kernels launched with PDL (1) or in plain stream order (0)
-extern int g_wide2d;  // 2D grids: single-pass stage kernels (1) or gather form (0)
-extern int g_seg1d;   // mixed 1D grids: staged-segment stage kernel (1) or gather form (0)
+extern int g_wide2d;  // 2D grids: step and single-pass stage kernels (1) or gather form (0)
+extern int g_seg1d;   // 1D grids: step kernel, FP64 segments above it (1) or the forms without (0)
 }
 namespace wide2d {
 extern int g_ty;  // 2D stage kernels' tile height: 0 = by grid size, else 8, 16 or 32
